@@ -671,7 +671,7 @@ def run_b200(args):
     except Exception as e:  # the checker library is optional on the bench path
         roofline["reference_kernel"] = {"unavailable": str(e)[:200]}
 
-    # the reference's own tuned W4A16 GEMM (oracle/_ref/libtm_ref_gemm*.so) next to ours on this model's four linears --
+    # the reference's own tuned W4A16 GEMM (oracle/_ref/libtm_ref_gemm_dd.so) next to ours on this model's four linears --
     # measurement only (B200_BENCH_REF_GEMM=0 switches it off)
     if os.environ.get("B200_BENCH_REF_GEMM", "0") != "0" and world == 1 and spec.weight_format == "awq":
         try:

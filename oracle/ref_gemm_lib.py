@@ -1,21 +1,16 @@
-"""TEST INFRASTRUCTURE -- ctypes binding of oracle/_ref/libtm_ref_gemm.so: the REFERENCE's own weight-only-quant GEMM
-(src/turbomind/kernels/gemm: gemm::Gemm::Run + the sm80 s16816 kernel family, weight repack through the reference's
-converters) compiled in place by oracle/ref_build/Makefile (kernel bodies from compute_80 PTX -> sm_100 SASS, see
-ref_gemm_shim.cu).
+"""TEST INFRASTRUCTURE -- ctypes binding of oracle/_ref/libtm_ref_gemm_dd.so: the REFERENCE's own weight-only-quant GEMM
+(src/turbomind/kernels/gemm: gemm::Gemm::Run + the sm80 s16816 kernel templates, weight repack through the reference's
+converters) compiled in place by oracle/ref_build/Makefile.
 
 Only tests/ and explicitly requested measurement legs may import this module; the product path (lmdeploy_b200/) never
-does.  The .so is built where /root/reference exists and travels to the GPU box with the repo snapshot."""
+does.  The .so is built where the reference's sources are and travels to the GPU with the built files."""
 import ctypes as C
 import os
 
 ROOT = os.path.dirname(os.path.abspath(__file__))
-# B200_REF_GEMM_LIB=ptx: the build whose kernel TUs hold compute_80 PTX only (JIT-compiled by the driver at load time, the way
-# the reference's wheels reach Blackwell); default: the ahead-of-time sm_100 SASS build of the same sources
-# default ("dd"): the reference's kernel templates registered with the evict-first L2 hint off (oracle/ref_build/
-# ref_gemm_kernels_dd.cu) -- the reference's own registration raises "illegal instruction" on a B200 with this toolchain;
-# "sass" = its own registration compiled ahead of time, "ptx" = the same through the driver JIT (both kept for the record)
-LIB_PATH = os.path.join(ROOT, "_ref", {"ptx": "libtm_ref_gemm_ptx.so", "sass": "libtm_ref_gemm.so"}.get(
-    os.environ.get("B200_REF_GEMM_LIB", "dd"), "libtm_ref_gemm_dd.so"))
+# The reference's kernel templates registered with the evict-first L2 hint off (oracle/ref_build/ref_gemm_kernels_dd.cu): its own
+# registration raises "illegal instruction" on a B200 with this toolchain and is neither built nor run.
+LIB_PATH = os.path.join(ROOT, "_ref", "libtm_ref_gemm_dd.so")
 DISPATCH_DEFAULT, DISPATCH_MEASURE, DISPATCH_REUSE = 0, 1, 2
 
 _lib = None

@@ -1,5 +1,5 @@
 """TEST INFRASTRUCTURE -- one TurboMind decode step assembled from the REFERENCE's OWN kernels compiled in place
-(oracle/_ref: libtm_ref_attention.so, libtm_ref_gemm.so, libtm_ref_norm.so), run in the order the reference runs them:
+(oracle/_ref: libtm_ref_attention.so, libtm_ref_gemm_dd.so, libtm_ref_norm.so), run in the order the reference runs them:
 
     LanguageModel::Impl::Forward     models/language_model.cc:493-542   embedding rows -> decoder -> lm_head
     UnifiedDecoder::Forward          models/llama/unified_decoder.cc:226-346

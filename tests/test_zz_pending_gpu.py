@@ -13,7 +13,7 @@ from test_linear_gpu import DevLinear, _assert_close
 pytestmark = [pytest.mark.gpu, pending_first_gpu_run]
 
 # ---------------------------------------------------------------------------------------------------------------
-# W4A16 linear against the REFERENCE's own GEMM (oracle/_ref/libtm_ref_gemm.so) on the same device buffers
+# W4A16 linear against the REFERENCE's own GEMM (oracle/_ref/libtm_ref_gemm_dd.so) on the same device buffers
 # ---------------------------------------------------------------------------------------------------------------
 @pytest.mark.parametrize("shape", [(4096, 4096), (4096, 6144), (14336, 4096)])
 @pytest.mark.parametrize("m", [1, 64])
@@ -24,7 +24,7 @@ def test_w4a16_matches_reference_gemm(lib, shape, m):
     import torch
     from oracle import ref_gemm_lib as RG
     if not RG.available():
-        pytest.skip("oracle/_ref/libtm_ref_gemm.so not built (needs the reference checkout at build time)")
+        pytest.skip("oracle/_ref/libtm_ref_gemm_dd.so not built (needs the reference checkout at build time)")
     from harness import to_dev_T, from_dev_T
     K, N = shape
     rng = np.random.default_rng(K + N + m)
@@ -47,7 +47,7 @@ def test_gated_silu_matches_reference_gemm(lib):
     import torch
     from oracle import ref_gemm_lib as RG
     if not RG.available():
-        pytest.skip("oracle/_ref/libtm_ref_gemm.so not built")
+        pytest.skip("oracle/_ref/libtm_ref_gemm_dd.so not built")
     from harness import to_dev_T, from_dev_T
     K, N, m = 4096, 2048, 32
     rng = np.random.default_rng(21)

@@ -1,4 +1,4 @@
-"""Development tool (measurement only): the reference's own W4A16 GEMM (oracle/_ref/libtm_ref_gemm.so -- gemm::Gemm::Run with
+"""Development tool (measurement only): the reference's own W4A16 GEMM (oracle/_ref/libtm_ref_gemm_dd.so -- gemm::Gemm::Run with
 its sm80 s16816 kernels, tuned per shape by its own measurer) timed next to ours on the decode shapes, both captured in a
 CUDA graph over rotating weight copies so every launch streams its weights from HBM.
 
@@ -102,7 +102,7 @@ def main():
     m = int(sys.argv[1]) if len(sys.argv) > 1 else 64
     iters = int(sys.argv[2]) if len(sys.argv) > 2 else 20
     if not RG.available():
-        print("oracle/_ref/libtm_ref_gemm.so is not built")
+        print("oracle/_ref/libtm_ref_gemm_dd.so is not built")
         return 1
     print(RG.load().ref_gemm_version().decode())
     measure(m, iters)
