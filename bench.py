@@ -1,9 +1,9 @@
 #!/usr/bin/env python
-"""bench.py -- decode tokens/s of the B200-native TurboMind decode path (BASELINE.json metric).
+"""bench.py -- decode tokens/s of the B200-native TurboMind decode path.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl b200|reference] [--config c2|c3|c1-tiny]
 
-Workload (BASELINE.json configs[1], "C2"): InternLM2-7B geometry, W4A16 AWQ (u4 g128) weights + KV int8, bs = 64,
+Workload ("C2"): InternLM2-7B geometry, W4A16 AWQ (u4 g128) weights + KV int8, bs = 64,
 2K context, greedy decode; synthetic random weights / KV (no checkpoints exist in the image).  A "step" is one
 decode forward for the whole batch (64 new tokens).  N > 1 = tensor parallel over N GPUs of one box (heads / FFN /
 vocab sharded, fused NVLink all-reduce), launched by torchrun, one rank per GPU: total work is fixed => "strong".
@@ -33,7 +33,7 @@ CONFIGS = {
     "c3": ("llama3-8b", 128, 4096, 4),
     "c4": ("internlm2-20b", 64, 2048, 0),
     "c1-tiny": ("internlm2-1.8b", 1, 128, 0),
-    # Llama-3-70B FP8 + KV-int8 at tensor-parallel 8 (BASELINE config 5): 70 GB of weights + 44 GB of KV, so it needs
+    # Llama-3-70B FP8 + KV-int8 at tensor-parallel 8: 70 GB of weights + 44 GB of KV, so it needs
     # --gpus >= 2; launch under torchrun with --gpus 8 for the configuration as named
     "c5": ("llama3-70b", 32, 8192, 8),
 }
@@ -328,7 +328,7 @@ class ClockSampler:
 
     Primary backend: NVML in this process (pynvml), one sample every 2 ms from a thread, so even a 50 ms timed region
     (TP8) holds tens of samples.  Fallback: `nvidia-smi -lms`, started by start() BEFORE the warm-up because the tool
-    takes about a second to come up on an 8-GPU box (an N=8 run of round 1 ended with zero samples that way).  Either
+    takes about a second to come up on an 8-GPU box (an eight-GPU run once ended with zero samples that way).  Either
     way only samples stamped inside [begin, end] of the `with` block count."""
 
     # NVML clocks-event-reason bits (nvml.h; stable ABI)

@@ -5,7 +5,7 @@
  * InternLM/lmdeploy 0.16.0 (paths relative to the reference root).  The reference has no extern "C"
  * surface (its FFI is the pybind11 module `_turbomind`, src/turbomind/python/bind.cpp:423-1004);
  * these are the plain-pointer equivalents of the *inner* operator boundary its own layers call
- * (SURVEY.md section 8b), plus an engine-level handle API that stands where
+ * plus an engine-level handle API that stands where
  * LanguageModel::Run / ModelRequest::Forward sit.  INTEGRATION.md shows the binding a maintainer adds.
  *
  * Conventions: all pointers are DEVICE pointers unless a name ends in `_host`; `stream` is a

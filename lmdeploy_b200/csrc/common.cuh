@@ -1,6 +1,6 @@
 // Device-side primitives shared by the sm_100a kernels: mbarrier, bulk async copy (TMA 1-D),
 // mma.sync fragments, sub-byte -> half/bf16 converters with the exact rounding contract of the
-// reference (see DESIGN.md "numerics contract").
+// reference.
 #pragma once
 
 #include <cuda_bf16.h>

@@ -16,7 +16,7 @@ namespace gemm {
 
 // ------------------------------------------------------------------------------------------------
 // prepare: loader-visible tensors -> tile stream consumed by gemm_kernel
-//   u4 input (pre-prepare format, SURVEY 8a11 / lmdeploy/turbomind/weight_format.py:63-74):
+//   u4 input (pre-prepare format, lmdeploy/turbomind/weight_format.py:63-74):
 //     qweight int32 [K, N/8], nibble i of word w = column 8w+i;  scales, zeros T [K/128, N]
 //   output per (n-tile nt, k-group kg):  data [c:2][hh:2][n:128][16 B] then params [n:128]{s, t=-z*s}
 //   the 32 nibbles of a 16-byte unit are k = kg*128 + c*64 + hh*32 + (0..31); inside each u32 the nibble
@@ -109,7 +109,7 @@ __global__ void u4_fast_flag_kernel(int* trailer)
     trailer[1] = 0;
 }
 
-// fp8 (e4m3 + 128x128 block scales, SURVEY 8a11 / linear_weight.cc:138-150): W u8 [K, N] (trans == 0) or [N, K]
+// fp8 (e4m3 + 128x128 block scales, linear_weight.cc:138-150): W u8 [K, N] (trans == 0) or [N, K]
 // (trans == 1), scale_inv f32 [K/128, N/128]  ->  per (nt, kg): data [k16:8][n:128][16 B], then the block scale cast to T
 template<class T>
 __global__ void prepare_fp8_kernel(uint8_t* dst, const uint8_t* w, const float* scale_inv, int K, int N, int trans)
@@ -273,7 +273,7 @@ static Plan make_plan(int fmt, int MT, int N, int K, bool need_split = false)
     }
     // Short K (<= 16 groups: the row-split wo / w2 of a tensor-parallel shard): one tile per CTA and NO split beats any
     // split plan -- the 4.3 us exchange costs more than the K-groups it saves (measured on the per-rank shapes of
-    // InternLM2-7B / 20B and Llama-3-70B at TP 2-8, profiles/r02_raw/gemm_sweep_*: e.g. K 1024, N 4096: 11.8 -> 5.3 us).
+    // InternLM2-7B / 20B and Llama-3-70B at TP 2-8: e.g. K 1024, N 4096: 11.8 -> 5.3 us).
     // (need_split: the fused residual + RMSNorm epilogue lives in the split-K exchange and keeps the split plan.)
     if (!need_split && fmt != kDense && ov.tiles == 0 && ov.splits == 0 && kgs <= 16 && N / kBN <= slots) {
         pl.tiles  = 1;

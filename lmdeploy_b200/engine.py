@@ -100,7 +100,7 @@ class StaticBatchRunner:
         """CUDA-event time of the decode attention at context k_len: decode_attention_kernel alone (prologue / fix-up
         skipped, the default) or -- full=True -- the whole b200_decode_attention call (prologue + main kernel + fix-up), which
         is what compares with the reference's dispatchDecoding (in-kernel prologue + its reduce).
-        Algorithmic bytes per launch = batch * k_len * 2 * Hkv * (D * kvbits / 8 + 4) (SURVEY 8d)."""
+        Algorithmic bytes per launch = batch * k_len * 2 * Hkv * (D * kvbits / 8 + 4)."""
         m = self.model
         spec = m.spec
         D = spec.head_dim
@@ -124,7 +124,7 @@ class StaticBatchRunner:
         p.quant_policy, p.dtype = m.quant_policy, m.cfg.dtype
         p.workspace, p.workspace_bytes = ws.data_ptr(), ws.numel()
         p.stream = torch.cuda.current_stream().cuda_stream
-        # main-kernel-only timing uses the round-1 three-kernel form (debug bit 2) with prologue and fix-up skipped (bits 0, 1):
+        # main-kernel-only timing uses the three-kernel form (debug bit 2) with prologue and fix-up skipped (bits 0, 1):
         # one unfused full call first leaves the rotated q it reads; full=True times the op as callers get it (one fused kernel)
         p.debug_flags = 0 if full else 4
         if full:

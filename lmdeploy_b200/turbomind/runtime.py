@@ -204,7 +204,7 @@ class DecodeModel:
             torch.cuda.synchronize()
 
     def load_synthetic(self, seed=0):
-        """Random weights of the real shapes (no checkpoints exist in the image)."""
+        """Random weights of the real shapes (no checkpoint needed)."""
         s = self.spec
         g = torch.Generator(device=self.device)
         g.manual_seed(seed * 1000 + self.tp_rank)
@@ -307,7 +307,7 @@ class DecodeModel:
             torch.cuda.synchronize()
             del kv
 
-    # algorithmic bytes (SURVEY 8d): weights + lm_head + KV read (+ write) for this rank
+    # algorithmic bytes: weights + lm_head + KV read (+ write) for this rank
     def step_bytes(self, batch, ctx):
         q_bits = 16 if self.quant_policy == 0 else self.quant_policy
         D = self.spec.head_dim

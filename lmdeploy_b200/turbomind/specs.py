@@ -1,4 +1,4 @@
-"""Model geometries on the hot path (SURVEY.md section 8; public HF configs of these models --
+"""Model geometries on the hot path (public HF configs of these models --
 lmdeploy/turbomind/models/internlm2.py:70-84, models/llama.py:44-99 read the same fields)."""
 from dataclasses import dataclass, replace
 

@@ -1,7 +1,7 @@
 """CPU oracle for the TurboMind decode hot path -- TEST INFRASTRUCTURE ONLY.
 
 This package is a numpy restatement of the reference algorithm (InternLM/lmdeploy
-0.16.0, src/turbomind) for the decode hot path named in BASELINE.json.  Each
+0.16.0, src/turbomind) for the decode hot path.  Each
 function cites the reference file:line it follows.
 
 Only ``tests/``, ``__graft_entry__.smoke()`` and ``bench.py``'s ``cpu_baseline`` /
@@ -10,7 +10,7 @@ CPU baseline.  Nothing under ``lmdeploy_b200/`` imports it; the product path
 fails loudly when the CUDA library is missing.
 
 Parity pinning: PINNED against the reference itself.  The reference stores no golden
-vectors for this path (SURVEY.md section 8c) and its build system cannot be configured
+vectors for this path and its build system cannot be configured
 offline, but its decode-attention translation units compile from their sources in place:
 oracle/ref_build/ builds them (unmodified, from /root/reference) into
 oracle/_ref/libtm_ref_attention.so, and

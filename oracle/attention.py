@@ -12,7 +12,7 @@ Restates, in numpy, the algorithm of
   src/turbomind/kernels/attention/impl_81616.h:510-617      (Softmax / ConvertStoP)
   src/turbomind/kernels/attention/reduce.cu:90-153          (split-K merge)
 
-Numerics contract (DESIGN.md): T-typed ops are single RNE-rounded ops; where the
+Numerics contract: T-typed ops are single RNE-rounded ops; where the
 reference's release build uses hardware approximations (ex2.approx / sin.approx /
 div.approx under --use_fast_math) the oracle -- and our CUDA kernels -- use the
 correctly rounded operation instead.
@@ -414,7 +414,7 @@ def process_kv(cache: PagedKvCache, block_table, layer, start, k, v, rope: RopeP
 # --------------------------------------------------------------------------------------
 def prefill_attention(qkv, cache: PagedKvCache, block_tables, q_lens, k_lens, layer, num_heads, num_kv_heads,
                       rope: RopeParam, inv_sqrt_dh=None, q_bias=None, k_bias=None, v_bias=None):
-    """Chunked causal prefill for one layer (SURVEY 8f rank 1): the reference writes the chunk's K/V into the pages
+    """Chunked causal prefill for one layer: the reference writes the chunk's K/V into the pages
     (ProcessKV_v2, kv_cache_utils_v2.cu:18-210), reads them back de-quantised (FlattenKV_v2) and runs causal attention
     over keys [0, history + i] for query i of the chunk (attention_universal.h:355-553 with the prefill mainloop;
     same softmax arithmetic as decode).

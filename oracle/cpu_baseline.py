@@ -2,7 +2,7 @@
 host core (test/bench infrastructure only -- never on the product path).
 
 BASELINE.json asks for "the reference's PyTorchEngine CPU path"; the reference has NO CPU engine
-(lmdeploy/messages.py:531 admits only cuda/ascend/maca/camb -- SURVEY.md section 0), so this is a port ("kind":
+(lmdeploy/messages.py:531 admits only cuda/ascend/maca/camb), so this is a port ("kind":
 "port") structured like PyTorchEngine's default-backend ops:
   * W4A16 linear = dequantise-then-matmul      lmdeploy/pytorch/backends/default/awq_modules.py:37-46
   * RMSNorm                                    lmdeploy/pytorch/backends/default/norm.py:14-27

@@ -1,8 +1,7 @@
 // TEST INFRASTRUCTURE, not product code.
 // Thin C-ABI shim around the REFERENCE's own weight-only-quant GEMM (compiled in place from /root/reference by
 // oracle/ref_build/Makefile into oracle/_ref/libtm_ref_gemm_dd.so; no reference source is copied into this repo), so that
-// bench / tools can time the unmodified TurboMind W4A16 path on the same B200 next to ours ("the kernel to
-// beat").  The reference's sm80 s16816 kernels have empty bodies when compiled natively for sm_100 (their Arch tag is
+// bench / tools can time the unmodified TurboMind W4A16 path on the same B200 next to ours.  The reference's sm80 s16816 kernels have empty bodies when compiled natively for sm_100 (their Arch tag is
 // [800, 900), gemm_universal.h:174-175); the Makefile therefore compiles the kernel translation units from compute_80
 // PTX to sm_100 SASS -- the same code the reference executes on Blackwell through the PTX JIT.
 //

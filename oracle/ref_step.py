@@ -8,7 +8,7 @@
     lm_head: dense T weights go to cuBLAS with fp32 compute (LlamaLinear.cu, cublas.cu:92-110) -> torch.matmul here
     greedy: argmax of the fp32-cast T logits (generation/generation.cc:270-276)
 
-This is SURVEY section 8c's "L2" protocol: greedy token ids of the product against a forward built from reference kernels
+This is the "L2" protocol: greedy token ids of the product against a forward built from reference kernels
 on the same synthetic weights and KV pages.  Two honest deviations, both outside the kernels under test:
   * the step's first RMSNorm (no residual add) is run through the reference's fused residual+RMSNorm kernel with a zero
     addend (x + 0 == x in T), because invokeRMSNorm takes core::Tensor arguments the shim does not build;

@@ -1,6 +1,6 @@
 """GPU parity: b200_decode_attention (C ABI) vs the CPU oracle on identical seeded inputs.
 
-Bars (DESIGN.md numerics contract):
+Bars:
   * KV-cache bytes written by the decode prologue (quantised k/v of the new token, their (scale, zero))
     -- BIT-EXACT vs the oracle.
   * attention output (fp16/bf16): |diff| <= 2e-3 abs for N(0,1) inputs (fp32 accumulation order and
@@ -89,7 +89,7 @@ def test_run_to_run_determinism():
 
 
 def test_full_size_sampled():
-    """BASELINE config 2 shape (bs=64, ctx 2048, 32 q heads / 8 kv heads, KV int8): cache written by
+    """Headline shape (bs=64, ctx 2048, 32 q heads / 8 kv heads, KV int8): cache written by
     b200_process_kv on the GPU, attention checked against the oracle on sampled (sequence, kv-head) pairs
     that read back the GPU-written pages; plus size-independent properties."""
     import ctypes as C
@@ -212,8 +212,8 @@ def test_fused_kernel_equals_the_three_kernel_form(kv_bits, dtype, flags):
 def test_partials_of_an_earlier_call_do_not_leak_into_a_sparse_one(flags):
     """A workspace that served a big call (every CTA of the grid left fp32 partials) then serves a small one whose tiles are
     fewer than the grid's CTAs: the pieces of a multi-tile sequence then sit in CTAs with EMPTY CTAs in between, whose
-    partial slots still hold the big call's values.  The merge must visit the pieces only (round 1 walked the whole CTA
-    range and was right only on a zeroed workspace)."""
+    partial slots still hold the big call's values.  The merge must visit the pieces only (walking the whole CTA
+    range is right only on a zeroed workspace)."""
     import ctypes as C
     import torch
     from lmdeploy_b200 import _lib as L

@@ -1,5 +1,5 @@
 """Whole decode steps beyond the C2 default: bf16 (dense / fp8 weights), synthetic fp8 model, q/k/v bias (Qwen2), odd GQA
-groups, per-head q/k RMSNorm (Qwen3) -- each against the oracle.  First device run: round 2."""
+groups, per-head q/k RMSNorm (Qwen3) -- each against the oracle."""
 import numpy as np
 import pytest
 
@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 
 # ---------------------------------------------------------------------------------------------------------------
-# whole decode step in bf16: fp8 weights (Llama-3-70B FP8 is BASELINE config C5) and dense bf16 weights
+# whole decode step in bf16: fp8 weights (Llama-3-70B FP8) and dense bf16 weights
 # ---------------------------------------------------------------------------------------------------------------
 @pytest.mark.parametrize("kv_bits", [8, 16])
 @pytest.mark.parametrize("fmt", ["fp8", "fp16"])

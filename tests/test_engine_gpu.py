@@ -1,5 +1,5 @@
 """Continuous-batching engine on a device: TurboMind.step through scheduler, block allocation, host marshalling, CUDA-graph
-replay per batch size, prefix caching, chunked prefill.  First device run: round 2."""
+replay per batch size, prefix caching, chunked prefill."""
 import numpy as np
 import pytest
 

@@ -1,5 +1,4 @@
-"""FP8-weight GEMM (weight_format 3: e4m3 + per-(128-k-group, column) scales, the form the loader emits) vs the numpy oracle.
-First device run: round 2 (profiles/r02_first_call.md)."""
+"""FP8-weight GEMM (weight_format 3: e4m3 + per-(128-k-group, column) scales, the form the loader emits) vs the numpy oracle."""
 import numpy as np
 import pytest
 

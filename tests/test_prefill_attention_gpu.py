@@ -1,5 +1,5 @@
 """tcgen05 prefill attention + the mixed prefill/decode step: vs the oracle and vs the reference's own kernels
-(ProcessKV + FlattenKV + dispatchAttention built in place, oracle/_ref/libtm_ref_prefill.so).  First device run: round 2."""
+(ProcessKV + FlattenKV + dispatchAttention built in place, oracle/_ref/libtm_ref_prefill.so)."""
 import numpy as np
 import pytest
 

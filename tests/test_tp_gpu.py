@@ -1,4 +1,4 @@
-"""Tensor-parallel decode step on REAL GPUs (needs >= 2 devices: `gpurun --gpus 2 -- python -m pytest tests -m gpu`):
+"""Tensor-parallel decode step on REAL GPUs (needs >= 2 devices: `python -m pytest tests -m gpu`):
 one process per GPU, CUDA-IPC peer buffers, the fused NVLink all-reduce + residual + RMSNorm kernel and the argmax
 exchange (csrc/comm.cu).  Checked against the same model run on ONE GPU through the same C ABI:
   * greedy token streams identical on every rank and equal to the single-GPU stream wherever the single-GPU
@@ -74,7 +74,7 @@ def test_tp2_decode_matches_single_gpu():
     import torch
     import torch.multiprocessing as mp
     if torch.cuda.device_count() < 2:
-        pytest.skip("needs 2 GPUs (gpurun --gpus 2)")
+        pytest.skip("needs 2 GPUs")
     from test_decode_step_gpu import build_device_model
     w = TinyWeights(hidden=512, layers=2, heads=4, kv_heads=2, inter=1024, vocab=1024, seed=11)
     m1 = build_device_model(w, 8, max_batch=B)

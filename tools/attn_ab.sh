@@ -5,7 +5,7 @@
 # experiment's outcome is in profiles/r02_attention_variants.md and the variants are not kept in the tree.
 set -u
 cd "$(dirname "$0")/.."
-mkdir -p gpurun_out
+
 L=$PWD/lmdeploy_b200/lib
 {
 for lib in libb200tm_head.so libb200tm_exactint.so libb200tm.so; do
@@ -16,4 +16,4 @@ for lib in libb200tm_head.so libb200tm_exactint.so libb200tm.so; do
 done
 B200_LIB_PATH=$L/libb200tm_head.so timeout 300 python tools/attn_ab.py 4 40 2>&1 | tail -n 1
 B200_LIB_PATH=$L/libb200tm.so timeout 300 python tools/attn_ab.py 4 40 2>&1 | tail -n 1
-} | tee gpurun_out/attn_ab.log
+} 

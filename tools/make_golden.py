@@ -1,10 +1,10 @@
 #!/usr/bin/env python
-"""Generates tests/golden/ref_attention_*.npz on a GPU box: inputs and outputs of the REFERENCE's own kernels
+"""Generates tests/golden/ref_attention_*.npz on a GPU: inputs and outputs of the REFERENCE's own kernels
 (oracle/_ref/libtm_ref_attention.so = TurboMind ProcessKV_v2 + dispatchDecoding built in place for sm_100a).
 The fixtures let the CPU test-suite (tests/test_golden_cpu.py) pin the numpy oracle to what the reference actually
-computes, without a GPU and without /root/reference.
+computes, without a GPU and without its sources.
 
-    gpurun -- 'python tools/make_golden.py && cp /tmp/golden/*.npz gpurun_out/'     (then move into tests/golden/)
+    python tools/make_golden.py <output folder>     (then move the files into tests/golden/)
 """
 import ctypes as C
 import os
@@ -99,7 +99,7 @@ def run_case(kv_bits, rope_name, out_dir):
 
 
 if __name__ == "__main__":
-    out_dir = sys.argv[1] if len(sys.argv) > 1 else os.path.join(ROOT, "gpurun_out", "golden")
+    out_dir = sys.argv[1] if len(sys.argv) > 1 else "golden"
     os.makedirs(out_dir, exist_ok=True)
     for kv_bits, rope_name in [(8, "default"), (4, "default"), (16, "default"), (8, "llama3")]:
         run_case(kv_bits, rope_name, out_dir)

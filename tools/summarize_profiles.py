@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""Summarise gpurun_out ncu artefacts into profiles/ (tracked).
+"""Summarise ncu artefacts into profiles/ (tracked).
   python tools/summarize_profiles.py launches <launches.csv> <out.md> [title]
   python tools/summarize_profiles.py rep <file.ncu-rep> <out.md> [title]
 """
