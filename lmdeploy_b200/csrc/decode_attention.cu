@@ -318,7 +318,9 @@ __global__ void __launch_bounds__(128) prefill_prologue_kernel(const ProloguePar
     pdl_launch_dependents();
     pdl_wait();
     if (blockIdx.x == 0) {
-        prefill_plan<128>(plan);
+        if (plan.partial) {
+            prefill_plan<128>(plan);
+        }
         return;
     }
     using Ops        = TypeOps<T>;
@@ -659,28 +661,31 @@ static int launch_decode(const b200_attention_params* a)
 // prefill: prologue (bias + RoPE + KV quantise/store + rotated Q) then the tcgen05 causal attention kernel
 // ------------------------------------------------------------------------------------------------
 struct PrefillWorkspace {
-    void*        q_rot;
-    PrefillUnit* units;
+    void*         q_rot;
+    PrefillUnit*  units;
     PrefillRange* ranges;
-    float*       partial;
-    size_t       least, total;  // without / with room for partials
+    float*        partial;
+    size_t        total;
 };
 
-static PrefillWorkspace carve_prefill(void* base, int token_num, int num_heads)
+// `bytes` < total: room for the rotated queries alone, everything else null
+static PrefillWorkspace carve_prefill(void* base, size_t bytes, int token_num, int num_heads)
 {
     PrefillWorkspace w{};
-    size_t           off = 0;
-    auto             take = [&](size_t bytes) {
+    size_t           off  = 0;
+    auto             take = [&](size_t n) {
         void* p = base ? (char*)base + off : nullptr;
-        off += align_up(bytes, 256);
+        off += align_up(n, 256);
         return p;
     };
     w.q_rot   = take((size_t)token_num * num_heads * kHeadDim * 2);
     w.units   = (PrefillUnit*)take(((size_t)token_num + 1) * sizeof(PrefillUnit));  // a unit holds at least one token
     w.ranges  = (PrefillRange*)take(kPfMaxCtas * sizeof(PrefillRange));
-    w.least   = off;
     w.partial = (float*)take((size_t)kPfMaxCtas * 2 * 2 * kPfPartialFloats * sizeof(float));
     w.total   = off;
+    if (bytes < w.total) {
+        w.units = nullptr, w.ranges = nullptr, w.partial = nullptr;
+    }
     return w;
 }
 
@@ -688,8 +693,8 @@ template<class T, int KVBITS>
 static int launch_prefill(const b200_attention_params* a)
 {
     cudaStream_t     st = (cudaStream_t)a->stream;
-    PrefillWorkspace w  = carve_prefill(a->workspace, a->token_num, a->num_heads);
-    if (!a->workspace || a->workspace_bytes < w.least) {
+    PrefillWorkspace w  = carve_prefill(a->workspace, a->workspace_bytes, a->token_num, a->num_heads);
+    if (!a->workspace || a->workspace_bytes < (size_t)a->token_num * a->num_heads * kHeadDim * 2) {
         return fail(B200_ERR_WORKSPACE, "workspace too small (see b200_prefill_attention_workspace_bytes)");
     }
     if (a->out_packed_mt > 0) {
@@ -729,8 +734,7 @@ static int launch_prefill(const b200_attention_params* a)
     p.units         = w.units;
     p.ranges        = w.ranges;
     p.main_ctas     = grid;
-    // a caller with room for q_rot and the units alone gets ranges that end at (unit, kv-head) boundaries: no partials
-    p.partial        = a->workspace_bytes >= w.total ? w.partial : nullptr;
+    p.partial       = w.partial;
     const int groups = (a->num_heads + 2 * a->num_kv_heads + kPfItems - 1) / kPfItems;
     launch_k(prefill_prologue_kernel<T, KVBITS>, dim3(1 + (unsigned)(((int64_t)a->token_num * groups + 3) / 4)), dim3(128), 0, st,
              prologue_params(a, w.q_rot), p);
@@ -821,7 +825,7 @@ extern "C" int b200_process_kv(const b200_attention_params* a)
 
 extern "C" size_t b200_prefill_attention_workspace_bytes(int token_num, int num_heads)
 {
-    return carve_prefill(nullptr, token_num, num_heads).total;
+    return carve_prefill(nullptr, 0, token_num, num_heads).total;
 }
 
 extern "C" int b200_prefill_attention(const b200_attention_params* a)

@@ -86,7 +86,7 @@ struct PrefillParams {
     PrefillUnit*  units;   // written by prefill_plan, one more than there are units
     PrefillRange* ranges;  // [main_ctas]
     int           main_ctas;
-    float*       partial;  // [2 * CTA][2 tiles] partials, or null: ranges end at (unit, kv-head) boundaries
+    float*       partial;  // [2 * CTA][2 tiles] partials, or null: whole (unit, kv-head) pieces are dealt out, without units and ranges
 };
 
 // Units and their places, by one block of THREADS threads; thread = sequence.
@@ -144,13 +144,13 @@ B200_DEVICE void prefill_plan(const PrefillParams& p)
         p.units[s_base.x] = PrefillUnit{s_base.y, 0, p.batch, 0, 0, 0, 0, 0};
     }
     __syncthreads();
-    // the ranges: equal numbers of places per CTA; without room for partials whole pieces are dealt out and u is the number of units
+    // the ranges: equal numbers of places per CTA
     const int       n_units = s_base.x;
     const long long total   = (long long)p.num_kv_heads * s_base.y;
     const int       ctas    = (int)min((long long)p.main_ctas, total);
     for (int c = tid; c < p.main_ctas; c += THREADS) {
         PrefillRange range{n_units, 0, 0, ctas, total, 0};
-        if (p.partial && c < ctas) {
+        if (c < ctas) {
             const long long at = total * c / ctas;
             int             lo = 0, hi = n_units;  // the last unit whose places (of all kv-heads) begin at or before `at`
             while (hi - lo > 1) {
@@ -187,16 +187,16 @@ struct PrefillSegment {
 struct PrefillWalk {
     const PrefillParams& p;
     PrefillUnit          unit;
-    int                  u, r, left;  // unit, place inside it, places left (whole pieces: next piece, -, number of pieces)
+    int                  u, r, left;  // unit, place inside it, places left; whole pieces: next piece, sequence, units of the earlier ones
     B200_DEVICE PrefillWalk(const PrefillParams& p_): p(p_)
     {
-        const PrefillRange range = p.ranges[blockIdx.x];
         if (p.partial) {
+            const PrefillRange range = p.ranges[blockIdx.x];
             u = range.u, r = range.r, left = range.count;
             unit = p.units[u];
         }
         else {
-            u = blockIdx.x, r = 0, left = range.u * p.num_kv_heads;
+            u = blockIdx.x, r = 0, left = 0;
         }
     }
     B200_DEVICE bool next(PrefillSegment& s)
@@ -217,18 +217,31 @@ struct PrefillWalk {
                 s.j0 = max(0, from - kPfStart);
                 s.j1 = to - kPfStart;
             } while (s.j1 <= s.j0);  // the range holds no key tile of the piece
+            s.b = unit.b, s.q0 = unit.q0, s.tok0 = unit.tok0, s.q_len = unit.q_len, s.hist = unit.hist;
         }
         else {
-            if (u >= left) {
-                return false;
+            // no list in the workspace: the pieces come in order, so the sequence of this one lies at or behind the last one's
+            const int TQ2 = 2 * (kPfRows / (p.num_heads / p.num_kv_heads)), at = u / p.num_kv_heads;
+            for (;; ++r) {
+                if (r >= p.batch) {
+                    return false;
+                }
+                s.tok0            = p.cu_q_len[r];
+                s.q_len           = p.cu_q_len[r + 1] - s.tok0;
+                const int n_units = (s.q_len + TQ2 - 1) / TQ2;
+                if (at < left + n_units) {
+                    break;
+                }
+                left += n_units;
             }
-            unit = p.units[u / p.num_kv_heads];
-            s.h  = u % p.num_kv_heads;
-            s.n  = unit.n - kPfStart;
+            s.b    = r;
+            s.q0   = (at - left) * TQ2;
+            s.hist = p.cu_k_len[r + 1] - p.cu_k_len[r] - s.q_len;
+            s.h    = u % p.num_kv_heads;
+            s.n    = (s.hist + min(s.q_len, s.q0 + TQ2) - 1) / kPfKeys + 1;
             s.j0 = 0, s.j1 = s.n;
             u += gridDim.x;
         }
-        s.b = unit.b, s.q0 = unit.q0, s.tok0 = unit.tok0, s.q_len = unit.q_len, s.hist = unit.hist;
         return true;
     }
 };

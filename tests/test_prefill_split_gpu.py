@@ -1,5 +1,5 @@
 """Prefill attention where its work list is cut: key tiles of 128 at their edges, a few tokens over a long history (many CTAs per piece), empty
-tiles, GQA groups that leave rows unused, and the form without room for partials."""
+tiles, GQA groups that leave rows unused, and the form for callers whose workspace holds the rotated queries alone."""
 import numpy as np
 import pytest
 
@@ -10,23 +10,20 @@ from test_prefill_attention_gpu import _prefill_case
 pytestmark = pytest.mark.gpu
 
 
-class _SmallWorkspace:
-    """The library with the smallest workspace the operator takes: q_rot, the units and the ranges of 160 CTAs."""
+class _Workspace:
+    """The library with a smaller workspace: `more` bytes beyond the rotated queries, the least that the operator takes."""
 
-    def __init__(self, lib):
-        self.lib = lib
+    def __init__(self, lib, more):
+        self.lib, self.more = lib, more
 
     def __getattr__(self, name):
         return getattr(self.lib, name)
 
     def b200_prefill_attention_workspace_bytes(self, tokens, heads):
-        def up(n):
-            return (n + 255) // 256 * 256
-
-        return up(tokens * heads * 256) + up((tokens + 1) * 32) + 160 * 32
+        return tokens * heads * 256 + self.more
 
 
-@pytest.mark.parametrize("room", [True, False])
+@pytest.mark.parametrize("more", [None, 0, 20000])
 @pytest.mark.parametrize("kv_bits,dtype,heads,q_lens,hists", [
     (8, F16, (8, 2), [127, 128, 129, 64, 65, 1], [0, 0, 0, 64, 63, 127]),
     (16, F16, (4, 1), [3, 40], [1500, 700]),
@@ -34,8 +31,8 @@ class _SmallWorkspace:
     (16, BF16, (7, 1), [19, 37, 300], [0, 128, 127]),
     (8, BF16, (2, 2), [257, 1], [255, 900]),
 ])
-def test_cut_work_matches_oracle(lib, kv_bits, dtype, heads, q_lens, hists, room):
-    got, ref, pool, ref_pool = _prefill_case(lib if room else _SmallWorkspace(lib), q_lens=q_lens, hists=hists, Hq=heads[0], Hkv=heads[1], kv_bits=kv_bits,
+def test_cut_work_matches_oracle(lib, kv_bits, dtype, heads, q_lens, hists, more):
+    got, ref, pool, ref_pool = _prefill_case(lib if more is None else _Workspace(lib, more), q_lens=q_lens, hists=hists, Hq=heads[0], Hkv=heads[1], kv_bits=kv_bits,
                                              dtype=dtype, seed=sum(q_lens))
     assert np.array_equal(pool, ref_pool)
     # P is rounded to T before P.V and the output is rounded to T (half an ulp each, 2^-12 / 2^-9 relative to values up to 4): as for the whole prompts
