@@ -121,7 +121,8 @@ typedef struct {
     int              quant_policy;
     int              dtype;
 
-    /* workspace: b200_decode_attention_workspace_bytes() bytes, 256-byte aligned.  Stands where
+    /* workspace: b200_decode_attention_workspace_bytes() bytes, 256-byte aligned; decode and prefill calls of all sizes may share
+     * one (of the largest size that any of them asks for).  Stands where
      * split_cnt / partial_O / partial_ML (unified_attention_layer.cc:220-224) stand in the reference.  Like the reference's
      * GEMM barriers it must be ZERO when first used (it holds the arrival counters of the in-kernel fix-up, which every
      * launch leaves at zero again; a call that plans internally also clears them). */

@@ -458,14 +458,20 @@ static size_t align_up(size_t x, size_t a)
     return (x + a - 1) / a * a;
 }
 
-constexpr int kMaxGridBound = 148 * 6 * 2;  // upper bound used to size the workspace (any B200-class part)
+// Upper bound used to size the workspace (any B200-class part); two CTAs under 148 * 6 * 2, which pay for the counters' bytes below.
+constexpr int kMaxGridBound = 148 * 6 * 2 - 2;
+
+// The first bytes of a workspace are the arrival counters of the decode kernel's in-kernel fix-up: zero on first use, left zero by every
+// launch.  They lie at the same place for every batch and head count, and the prefill operator leaves them alone, so that calls of both
+// kinds and of every size may share one workspace.
+constexpr size_t kCounterBytes = (kMaxGridBound * 4 + 255) / 256 * 256;
 
 struct Workspace {
+    int*   seg_counters;
     void*  q_rot;
     float* partial_O;
     float* partial_ML;
     int*   plan;
-    int*   seg_counters;
     size_t total;
 };
 
@@ -478,14 +484,12 @@ static Workspace carve(void* base, int token_num, int batch, int num_heads)
         off += align_up(bytes, 256);
         return p;
     };
-    w.q_rot      = take((size_t)token_num * num_heads * kHeadDim * 2);
-    w.partial_O  = (float*)take((size_t)2 * kMaxGridBound * kMaxGroup * kHeadDim * 4);
-    w.partial_ML = (float*)take((size_t)2 * kMaxGridBound * kMaxGroup * 2 * 4);
-    w.plan       = (int*)take((size_t)(batch + 1) * 4);
-    // arrival counters of the in-kernel fix-up, one per (sequence, kv-head): must be zero on first use (the kernel re-arms
-    // them; the op's own plan launch clears them as well); sized for the largest kv-head count per group size 1
-    w.seg_counters = (int*)take((size_t)batch * num_heads * 4);
-    w.total      = off;
+    w.seg_counters = (int*)take(kCounterBytes);
+    w.q_rot        = take((size_t)token_num * num_heads * kHeadDim * 2);
+    w.partial_O    = (float*)take((size_t)2 * kMaxGridBound * kMaxGroup * kHeadDim * 4);
+    w.partial_ML   = (float*)take((size_t)2 * kMaxGridBound * kMaxGroup * 2 * 4);
+    w.plan         = (int*)take((size_t)(batch + 1) * 4);
+    w.total        = off;
     return w;
 }
 
@@ -590,7 +594,7 @@ static int launch_decode(const b200_attention_params* a)
     const int* plan = a->plan;
     if (!plan) {
         launch_k(plan_kernel, dim3(1), dim3(256), 0, st, w.plan, a->cu_k_len, a->finished, a->batch_size, w.seg_counters,
-                 a->batch_size * a->num_kv_heads);
+                 kMaxGridBound);
         if (int e = check_launch("plan_kernel")) {
             return e;
         }
@@ -668,7 +672,7 @@ struct PrefillWorkspace {
     size_t        total;
 };
 
-// `bytes` < total: room for the rotated queries alone, everything else null
+// `bytes` < total: room for the rotated queries alone (kept off the counters if that fits), everything else null
 static PrefillWorkspace carve_prefill(void* base, size_t bytes, int token_num, int num_heads)
 {
     PrefillWorkspace w{};
@@ -678,12 +682,15 @@ static PrefillWorkspace carve_prefill(void* base, size_t bytes, int token_num, i
         off += align_up(n, 256);
         return p;
     };
-    w.q_rot   = take((size_t)token_num * num_heads * kHeadDim * 2);
+    const size_t q_bytes = (size_t)token_num * num_heads * kHeadDim * 2;
+    take(kCounterBytes);  // the decode operator's, see there
+    w.q_rot   = take(q_bytes);
     w.units   = (PrefillUnit*)take(((size_t)token_num + 1) * sizeof(PrefillUnit));  // a unit holds at least one token
     w.ranges  = (PrefillRange*)take(kPfMaxCtas * sizeof(PrefillRange));
     w.partial = (float*)take((size_t)kPfMaxCtas * 2 * 2 * kPfPartialFloats * sizeof(float));
     w.total   = off;
     if (bytes < w.total) {
+        w.q_rot = bytes < kCounterBytes + q_bytes ? base : w.q_rot;
         w.units = nullptr, w.ranges = nullptr, w.partial = nullptr;
     }
     return w;

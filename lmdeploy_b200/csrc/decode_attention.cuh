@@ -265,7 +265,7 @@ struct KernelParams {
     const int*     readonly_block_num;
     const float2*  rope_table;
     RopeConst      rope;
-    int*           seg_counters;  // [batch * Hkv] arrivals per straddling segment; zero on entry, left zero
+    int*           seg_counters;  // [grid] arrivals per straddling segment, by the first CTA that has keys of it; zero on entry, left zero
     int            grid_main;
     int            early;  // the producer warp streams KV tiles before griddepcontrol.wait (see the kernel's head)
 };
@@ -354,7 +354,7 @@ struct WorkIter {
 // The main-kernel CTAs that hold a piece of segment (sequence b, kv-head h).  CTA c owns units [total * c / grid,
 // total * (c + 1) / grid).  With total >= grid every CTA is non-empty and the pieces sit in CTAs cf..cl; with total < grid a
 // CTA holds at most ONE unit (= one tile), empty CTAs lie in between, and the pieces are the segment's `tiles` units, unit
-// u living in CTA ((u + 1) * grid - 1) / total.  (Round 1 walked cf..cl in both cases and read the never-written -- or,
+// u living in CTA ((u + 1) * grid - 1) / total.  (Walking cf..cl in both cases would read the never-written -- or,
 // worse, stale -- partial slots of the empty CTAs in between.)
 struct SegCtas {
     int       cf, cl, first_slot, n;  // n = number of pieces
@@ -1317,7 +1317,7 @@ __global__ void __launch_bounds__(kThreads, min_ctas_per_sm<KVBITS>()) decode_at
                 named_bar_sync(1, kConsumerWarps * 32);
                 if (ctid == 0) {
                     ss.seg        = segment_ctas(p, it.b, it.h, p.grid_main);
-                    int*      ctr = p.seg_counters + it.b * Hkv + it.h;
+                    int*      ctr = p.seg_counters + ss.seg.cf;  // one segment at most leaves a CTA at its range's end
                     const int old = atom_add_acq_rel_gpu(ctr, 1);
                     ss.fix_last   = (old == ss.seg.n - 1);
                     if (old == ss.seg.n - 1) {
