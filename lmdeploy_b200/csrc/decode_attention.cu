@@ -711,13 +711,15 @@ static int launch_prefill(const b200_attention_params* a)
     if (G > kPfRows) {
         return fail(B200_ERR_UNSUPPORTED, "GQA group size > 128");
     }
-    auto             kern = prefill_attention_kernel<T, KVBITS>;
+    auto             kern = w.partial ? prefill_attention_kernel<T, KVBITS, true> : prefill_attention_kernel<T, KVBITS, false>;
     static PerDevice grids{};  // per (T, KVBITS) instantiation and per device
     const int        dev  = current_device();
     int              grid = grids.value[dev].load(std::memory_order_acquire);
     if (grid == 0) {
-        if (cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kPfSmem<KVBITS>); e != cudaSuccess) {
-            return fail_cuda(e, "cudaFuncSetAttribute(prefill_attention_kernel)");
+        for (auto k : {prefill_attention_kernel<T, KVBITS, true>, prefill_attention_kernel<T, KVBITS, false>}) {
+            if (cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kPfSmem<KVBITS>); e != cudaSuccess) {
+                return fail_cuda(e, "cudaFuncSetAttribute(prefill_attention_kernel)");
+            }
         }
         int sms = 0;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

@@ -29,21 +29,17 @@
 #pragma once
 
 #include "common.cuh"
+#include "prefill_work.cuh"
 #include "umma.cuh"
 
 namespace b200 {
 namespace attn {
 
-constexpr int kPfRows     = 128;  // UMMA M: query rows per tile
-constexpr int kPfKeys     = 128;  // keys per tile: UMMA N of S, K extent of P.V
-constexpr int kPfD        = 128;
-constexpr int kPfLoaders  = 7;    // warps that fill the K/V rings (16 warps in all: 128 registers a thread at launch)
-constexpr int kPfThreads  = 32 * (8 + 1 + kPfLoaders);
+constexpr int kPfThreads  = 32 * (8 + 1 + kPfLoaders);  // 16 warps: 128 registers a thread at launch
 constexpr int kPfTile     = kPfKeys * kPfD * 2;  // bytes of a Q, K or V operand tile
 constexpr int kPfStages   = 2;
-constexpr int kPfMaxCtas  = 160;  // bound of the persistent grid (sizes the partial buffers)
 constexpr int kPfColS = 0, kPfColO = 256, kPfTmemCols = 512;  // tile t: S / P at t * 128, O at 256 + t * 128
-constexpr int kPfStart    = 2;    // places that a piece takes in the work list before its key tiles (Q load, first scores, output)
+
 constexpr float kPfLazy   = 8.f;  // log2 of the growth of a row's maximum that forces a rescale
 
 // dynamic shared memory: Q tiles, K and V rings, and the staging tiles of quantised pages
@@ -53,42 +49,6 @@ constexpr int kPfSmem = (2 + 2 * kPfStages) * kPfTile + (KVBITS == 16 ? 0 : 2 * 
 // partial of one (CTA range end, tile): accumulator [d/4][row] float4, then (max, sum) [row] float2
 constexpr size_t kPfPartialFloats = (size_t)kPfRows * kPfD + 2 * kPfRows;
 
-struct alignas(16) PrefillUnit {
-    int prefix;       // places of all earlier units in the work list (one kv-head): kPfStart, then one per 128-key tile
-    int n;            // its own places
-    int b, q0;        // sequence, first query token of the unit inside the chunk
-    int tok0, q_len;  // the sequence's first token of the step and number of tokens
-    int hist, pad;
-};
-
-// where a CTA's range of the work list begins, and the whole list's length; written by prefill_plan
-struct alignas(16) PrefillRange {
-    int u, r;       // unit, place inside it (all kv-heads)
-    int count;      // places of the range
-    int ctas;       // ranges in all
-    long long total, pad;
-};
-
-struct PrefillParams {
-    const void* q_rot;  // [token][Hq][D], bias + RoPE applied (prologue kernel)
-    void*       out;    // [token][Hq*D]
-    int64_t     out_stride;
-    char**      block_ptrs;
-    const int*  cu_block_nums;
-    const int*  cu_q_len;
-    const int*  cu_k_len;
-    int         layer_offset;
-    int         block_len;
-    int         batch;
-    int         num_heads;
-    int         num_kv_heads;
-    float       qk_scale;  // log2(e) / sqrt(D)
-    PrefillUnit*  units;   // written by prefill_plan, one more than there are units
-    PrefillRange* ranges;  // [main_ctas]
-    int           main_ctas;
-    float*       partial;  // [2 * CTA][2 tiles] partials, or null: whole (unit, kv-head) pieces are dealt out, without units and ranges
-};
-
 // Units and their places, by one block of THREADS threads; thread = sequence.
 template<int THREADS>
 B200_DEVICE void prefill_plan(const PrefillParams& p)
@@ -96,7 +56,7 @@ B200_DEVICE void prefill_plan(const PrefillParams& p)
     __shared__ int2 s_warp[THREADS / 32];
     __shared__ int2 s_base;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int TQ2 = 2 * (kPfRows / (p.num_heads / p.num_kv_heads));
+    const int TQ2 = prefill_unit_tokens(p);
     if (tid == 0) {
         s_base = make_int2(0, 0);
     }
@@ -112,7 +72,7 @@ B200_DEVICE void prefill_plan(const PrefillParams& p)
         int2 v = make_int2(0, 0);  // (units, places)
         for (int q0 = 0; q0 < q_len; q0 += TQ2) {
             v.x += 1;
-            v.y += kPfStart + (hist + min(q_len, q0 + TQ2) - 1) / kPfKeys + 1;
+            v.y += prefill_places(hist, q_len, q0, TQ2);
         }
         int2 s = v;  // inclusive scan
 #pragma unroll
@@ -130,7 +90,7 @@ B200_DEVICE void prefill_plan(const PrefillParams& p)
         for (int w = 0; w < warp; ++w) base.x += s_warp[w].x, base.y += s_warp[w].y;
         int u = base.x + s.x - v.x, t = base.y + s.y - v.y;
         for (int q0 = 0; q0 < q_len; q0 += TQ2) {
-            const int n  = kPfStart + (hist + min(q_len, q0 + TQ2) - 1) / kPfKeys + 1;
+            const int n  = prefill_places(hist, q_len, q0, TQ2);
             p.units[u++] = PrefillUnit{t, n, b, q0, tok0, q_len, hist, 0};
             t += n;
         }
@@ -144,107 +104,10 @@ B200_DEVICE void prefill_plan(const PrefillParams& p)
         p.units[s_base.x] = PrefillUnit{s_base.y, 0, p.batch, 0, 0, 0, 0, 0};
     }
     __syncthreads();
-    // the ranges: equal numbers of places per CTA
-    const int       n_units = s_base.x;
-    const long long total   = (long long)p.num_kv_heads * s_base.y;
-    const int       ctas    = (int)min((long long)p.main_ctas, total);
     for (int c = tid; c < p.main_ctas; c += THREADS) {
-        PrefillRange range{n_units, 0, 0, ctas, total, 0};
-        if (c < ctas) {
-            const long long at = total * c / ctas;
-            int             lo = 0, hi = n_units;  // the last unit whose places (of all kv-heads) begin at or before `at`
-            while (hi - lo > 1) {
-                const int mid = (lo + hi) >> 1;
-                if ((long long)p.num_kv_heads * p.units[mid].prefix <= at) {
-                    lo = mid;
-                }
-                else {
-                    hi = mid;
-                }
-            }
-            range.u     = lo;
-            range.r     = (int)(at - (long long)p.num_kv_heads * p.units[lo].prefix);
-            range.count = (int)(total * (c + 1) / ctas - at);
-        }
-        p.ranges[c] = range;
+        p.ranges[c] = prefill_range(p, s_base.x, s_base.y, c);
     }
 }
-
-// One (unit, kv-head) piece: key tiles [j0, j1) of n
-struct PrefillSegment {
-    int b, q0, h, j0, j1, n;
-    int q_len, hist, tok0;
-    // tile t: valid query tokens and key tiles of it inside [j0, j1)
-    B200_DEVICE int tokens(int t, int TQ) const { return max(0, min(TQ, q_len - q0 - t * TQ)); }
-    B200_DEVICE int tiles(int t, int TQ) const
-    {
-        const int nq = tokens(t, TQ);
-        return nq ? max(0, min(j1, (hist + q0 + t * TQ + nq - 1) / kPfKeys + 1) - j0) : 0;
-    }
-};
-
-// walks the pieces of one CTA; every role of the CTA walks the same ones
-struct PrefillWalk {
-    const PrefillParams& p;
-    PrefillUnit          unit;
-    int                  u, r, left;  // unit, place inside it, places left; whole pieces: next piece, sequence, units of the earlier ones
-    B200_DEVICE PrefillWalk(const PrefillParams& p_): p(p_)
-    {
-        if (p.partial) {
-            const PrefillRange range = p.ranges[blockIdx.x];
-            u = range.u, r = range.r, left = range.count;
-            unit = p.units[u];
-        }
-        else {
-            u = blockIdx.x, r = 0, left = 0;
-        }
-    }
-    B200_DEVICE bool next(PrefillSegment& s)
-    {
-        if (p.partial) {
-            do {
-                if (left <= 0) {
-                    return false;
-                }
-                if (r >= p.num_kv_heads * unit.n) {
-                    unit = p.units[++u];
-                    r    = 0;
-                }
-                s.h            = r / unit.n;
-                const int from = r - s.h * unit.n, to = min(unit.n, from + left);
-                left -= to - from, r += to - from;
-                s.n  = unit.n - kPfStart;
-                s.j0 = max(0, from - kPfStart);
-                s.j1 = to - kPfStart;
-            } while (s.j1 <= s.j0);  // the range holds no key tile of the piece
-            s.b = unit.b, s.q0 = unit.q0, s.tok0 = unit.tok0, s.q_len = unit.q_len, s.hist = unit.hist;
-        }
-        else {
-            // no list in the workspace: the pieces come in order, so the sequence of this one lies at or behind the last one's
-            const int TQ2 = 2 * (kPfRows / (p.num_heads / p.num_kv_heads)), at = u / p.num_kv_heads;
-            for (;; ++r) {
-                if (r >= p.batch) {
-                    return false;
-                }
-                s.tok0            = p.cu_q_len[r];
-                s.q_len           = p.cu_q_len[r + 1] - s.tok0;
-                const int n_units = (s.q_len + TQ2 - 1) / TQ2;
-                if (at < left + n_units) {
-                    break;
-                }
-                left += n_units;
-            }
-            s.b    = r;
-            s.q0   = (at - left) * TQ2;
-            s.hist = p.cu_k_len[r + 1] - p.cu_k_len[r] - s.q_len;
-            s.h    = u % p.num_kv_heads;
-            s.n    = (s.hist + min(s.q_len, s.q0 + TQ2) - 1) / kPfKeys + 1;
-            s.j0 = 0, s.j1 = s.n;
-            u += gridDim.x;
-        }
-        return true;
-    }
-};
 
 B200_DEVICE void sts128(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d)
 {
@@ -282,19 +145,15 @@ struct PrefillKeyTile {
     }
 };
 
-// Loader warps: the 16-byte units of 128 token rows of K or of V.  A warp instruction takes 8 rows x 4 units (64 contiguous bytes per
-// row); the 8 lanes that store one 8-dim chunk write 128 contiguous bytes of the operand tile (no bank conflicts).
+// Loader warps: rows of K or of V (PrefillRowMap says which)
 template<class T, int KVBITS>
-struct PrefillRows {
-    static constexpr int kRow   = kPfD * KVBITS / 8;
-    static constexpr int kUnits = kRow / 16;                               // 16 / 8 / 4 per row
-    static constexpr int kInstr = kPfKeys / 8 * (kUnits / 4);              // warp instructions per tile
-    static constexpr int kIter  = (kInstr + kPfLoaders - 1) / kPfLoaders;  // 10 / 5 / 3 per warp
+struct PrefillRows: PrefillRowMap<KVBITS> {
+    using Map = PrefillRowMap<KVBITS>;
+    using Map::half_of;
+    using Map::key_of;
+    using Map::unit_of;
+    static constexpr int kRow = Map::kRow, kInstr = Map::kInstr, kIter = Map::kIter;
     uint32_t par[kIter];  // quantised pages: (scale, zero) of the thread's rows
-
-    B200_DEVICE static int key_of(int w, int lane, int it) { return (w + kPfLoaders * it) / (kUnits / 4) * 8 + (lane & 7); }
-    B200_DEVICE static int unit_of(int w, int lane, int it) { return (w + kPfLoaders * it) % (kUnits / 4) * 4 + (lane >> 3); }
-    B200_DEVICE static int half_of(int w, int it) { return (w + kPfLoaders * it) / (kUnits / 4) >> 3; }  // warp-uniform: key >> 6
 
     // asynchronous 16-byte copies of the tile's rows: T pages straight into the operand tile `dst`, quantised ones into the staging
     // tile `dst`, where instruction i of the tile has 512 bytes of its own
@@ -308,7 +167,7 @@ struct PrefillRows {
             const int      row  = key_of(w, lane, it), unit = unit_of(w, lane, it);
             const bool     live = x.j * kPfKeys + row <= x.last, half = half_of(w, it);
             const char*    src  = (half ? x.data1 : x.data0) + is_v * p.block_len * kRow + (live ? (row & 63) * kRow : 0) + unit * 16;
-            const uint32_t to   = KVBITS == 16 ? dst + unit * (kPfKeys * 16) + row * 16 : dst + (w + kPfLoaders * it) * 512 + lane * 16;
+            const uint32_t to   = KVBITS == 16 ? dst + Map::chunk_offset(unit, row) : dst + (w + kPfLoaders * it) * 512 + lane * 16;
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(src), "r"(live ? 16 : 0) : "memory");
             if constexpr (KVBITS != 16) {
                 par[it] = live ? *reinterpret_cast<const uint32_t*>((half ? x.param1 : x.param0) + is_v * p.block_len * 4 + (row & 63) * 4) : 0u;
@@ -326,7 +185,7 @@ struct PrefillRows {
                 break;
             }
             const uint4    raw = lds128(staging + (w + kPfLoaders * it) * 512 + lane * 16);
-            const uint32_t dst = tile + key_of(w, lane, it) * 16;
+            const uint32_t dst = tile + Map::chunk_offset(0, key_of(w, lane, it));
             const int      c0  = unit_of(w, lane, it) * (16 / KVBITS);  // first 8-dim chunk of the unit
             const uint32_t s2 = __byte_perm(par[it], par[it], 0x1010), z2 = __byte_perm(par[it], par[it], 0x3232);
 #pragma unroll
@@ -348,7 +207,9 @@ struct PrefillRows {
     }
 };
 
-template<class T, int KVBITS>
+// SPLIT: p.partial is there; else whole pieces (a kernel of its own: both walks in one cost registers, 178 -> 190 us on the
+// prompts above)
+template<class T, int KVBITS, bool SPLIT>
 __global__ void __launch_bounds__(kPfThreads, 1) prefill_attention_kernel(const PrefillParams p)
 {
     using Ops = TypeOps<T>;
@@ -385,8 +246,8 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attention_kernel(const 
     const uint32_t tmem = s_tmem;
     const uint32_t q_op = smem_u32(pf_smem), k_op = q_op + 2 * kPfTile, v_op = k_op + kPfStages * kPfTile;
 
-    PrefillWalk    walk(p);
-    PrefillSegment s;
+    PrefillWalk<SPLIT> walk(p, blockIdx.x);
+    PrefillSegment     s{};
 
     if (warp > 8) {
         // ================================ loaders ================================
@@ -605,7 +466,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attention_kernel(const 
             const int    pos_q = valid ? pos0 + tq : 0x7fffffff;  // padding rows see everything (finite softmax, never stored)
             const size_t tok   = (size_t)s.tok0 + s.q0 + t * TQ + tq;
             const int    h = s.h, j0 = s.j0;
-            const bool   whole = s.j0 == 0 && s.j1 == s.n;
+            const bool   whole = !SPLIT || (s.j0 == 0 && s.j1 == s.n);
             float        m = -INFINITY, l = 0.f;
             for (int i = 0; i < cnt; ++i) {
                 const int  key0 = (j0 + i) * kPfKeys;
@@ -706,9 +567,8 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attention_kernel(const 
                 }
             }
             else if (nq > 0) {
-                // ---- part of a piece: the CTA's first one if it began in an earlier CTA (slot 0), else its last one (slot 1) ----
-                const int slot = 2 * blockIdx.x + (j0 > 0 ? 0 : 1);
-                float*    dst  = p.partial + ((size_t)slot * 2 + t) * kPfPartialFloats;
+                // ---- part of a piece ----
+                float* dst = p.partial + ((size_t)prefill_slot(blockIdx.x, j0) * 2 + t) * kPfPartialFloats;
                 if (cnt > 0) {
 #pragma unroll 1
                     for (int ch = 0; ch < kPfD / 32; ++ch) {
@@ -742,22 +602,13 @@ __global__ void __launch_bounds__(kPfMergeThreads) prefill_merge_kernel(const Pr
     using Ops = TypeOps<T>;
     pdl_launch_dependents();
     pdl_wait();
-    const int          t = blockIdx.y, first = blockIdx.x + 1;
-    const PrefillRange range = p.ranges[first];  // grid.x = main_ctas - 1
-    if (first >= range.ctas) {
+    const int    t = blockIdx.y;
+    PrefillParts x;
+    if (!prefill_parts(p, blockIdx.x + 1, x)) {  // grid.x = main_ctas - 1
         return;
     }
-    const PrefillUnit unit = p.units[range.u];
-    const int         n    = unit.n, h = range.r / n, from = range.r - h * n;
-    if (from <= kPfStart) {
-        return;  // the range begins with the piece
-    }
-    // the list's places of the piece's first and last key tile, and their CTAs (CTA c begins at place total * c / ctas)
-    const long long s0 = (long long)p.num_kv_heads * unit.prefix + (long long)h * n + kPfStart, s1 = s0 + n - kPfStart - 1;
-    const int       cf = (int)(((s0 + 1) * range.ctas - 1) / range.total), cl = (int)(((s1 + 1) * range.ctas - 1) / range.total);
-    if (cf + 1 != first) {
-        return;  // an earlier block has it
-    }
+    const PrefillUnit unit = x.unit;
+    const int         h = x.h, cf = x.cf, cl = x.cl;
     const int G = p.num_heads / p.num_kv_heads, TQ = kPfRows / G;
     const int r = threadIdx.x & 127, tq = r / G, g = r - tq * G;
     if (tq >= TQ || unit.q0 + t * TQ + tq >= unit.q_len) {
@@ -776,8 +627,7 @@ __global__ void __launch_bounds__(kPfMergeThreads) prefill_merge_kernel(const Pr
         for (int i = 0; i < kBatch; ++i) {
             ml[i] = make_float2(-INFINITY, 0.f);
             if (cta + i <= cl) {
-                // only CTA cf's range begins at or before the piece: it left its part in its second slot, the others in their first
-                const float* part = p.partial + ((size_t)(2 * (cta + i) + (cta + i == cf ? 1 : 0)) * 2 + t) * kPfPartialFloats;
+                const float* part = p.partial + ((size_t)x.slot(cta + i) * 2 + t) * kPfPartialFloats;
                 ml[i]   = __ldcg(reinterpret_cast<const float2*>(part + (size_t)kPfRows * kPfD) + r);
                 v[i][0] = __ldcg(reinterpret_cast<const float4*>(part) + c0 * kPfRows + r);
                 v[i][1] = __ldcg(reinterpret_cast<const float4*>(part) + (c0 + 1) * kPfRows + r);
@@ -797,13 +647,13 @@ __global__ void __launch_bounds__(kPfMergeThreads) prefill_merge_kernel(const Pr
         }
     }
     const float inv = 1.f / L;
-    uint4       x;
-    x.x = Ops::pack2(o[0] * inv, o[1] * inv);
-    x.y = Ops::pack2(o[2] * inv, o[3] * inv);
-    x.z = Ops::pack2(o[4] * inv, o[5] * inv);
-    x.w = Ops::pack2(o[6] * inv, o[7] * inv);
+    uint4       y;
+    y.x = Ops::pack2(o[0] * inv, o[1] * inv);
+    y.y = Ops::pack2(o[2] * inv, o[3] * inv);
+    y.z = Ops::pack2(o[4] * inv, o[5] * inv);
+    y.w = Ops::pack2(o[6] * inv, o[7] * inv);
     *reinterpret_cast<uint4*>(reinterpret_cast<T*>(p.out) + ((size_t)unit.tok0 + unit.q0 + t * TQ + tq) * p.out_stride
-                              + ((size_t)h * G + g) * kPfD + c0 * 4) = x;
+                              + ((size_t)h * G + g) * kPfD + c0 * 4) = y;
 }
 
 }  // namespace attn

@@ -1,28 +1,35 @@
-"""Index-level emulation of csrc/prefill_attention.cuh on the CPU, checked against the independent oracle.
+"""The arithmetic and the operand addresses of csrc/prefill_attention.cuh, followed on the CPU and checked against the independent oracle.
 
-The kernel has not run on a device yet; what CAN be checked without one is everything that is not
-tensor-core semantics: the CTA -> (sequence, query tile) map, the row -> (token, head) stacking, page addressing (data and
-parameter regions, int4 nibble order), the operand-tile byte addresses (Q [d/8][row][8], K [d/8][key][8], V transposed
-[key/8][d][8] with its byte_perm selectors), tile count, causal mask, dead-key zeroing and the online-softmax recurrence.
-The emulation below follows the CUDA source statement by statement with the same names; the two tcgen05.mma groups are
-replaced by a generic reader of the UMMA canonical K-major layout (element (row, k) at (k/8)*LBO + (row/8)*SBO +
-(row%8)*16 + (k%8)*2 -- the layout tools/umma_probe.cu verified on hardware) followed by a float64 matmul."""
+Units of two tiles of 128 rows (row -> (token, head) stacking), page addressing (data and parameter regions, int4 nibble order) by the loaders' map of
+16-byte units, the operand tiles' byte addresses (Q [d/8][row][8]; K and V alike [d/8][key][8]: K-major operand of Q.K^T, MN-major operand of P.V), key
+tiles of 128 per tile of rows, causal mask, dead-key zeroing, online softmax, and the partials of a piece whose keys lie in several ranges, combined in
+order.  The tcgen05.mma groups are replaced by readers of the UMMA canonical layouts (no swizzle; tools/umma_probe.cu verified them on hardware) followed
+by a float64 matmul.  How the ranges are cut is checked on the kernels' own code in test_prefill_work_cpu.py."""
 import numpy as np
 import pytest
 
 from oracle import attention as OA
 from oracle.numerics import F16, from_bits, rn, to_bits
 
-ROWS, KEYS, D = 128, 64, 128
+ROWS, KEYS, D, LOADERS, START = 128, 128, 128, 7, 2
 
 
 def read_operand(buf, rows, ks, lbo, sbo):
     """UMMA canonical K-major, no swizzle: -> float32 [rows, ks] from a uint8 buffer."""
     r = np.arange(rows)[:, None]
     k = np.arange(ks)[None, :]
-    addr = (k // 8) * lbo + (r // 8) * sbo + (r % 8) * 16 + (k % 8) * 2
-    bits = buf[addr].astype(np.uint16) | (buf[addr + 1].astype(np.uint16) << 8)
-    return from_bits(bits, F16)
+    return _halves(buf, (k // 8) * lbo + (r // 8) * sbo + (r % 8) * 16 + (k % 8) * 2)
+
+
+def read_mn_major(buf, n, ks, k_stride, n_stride):
+    """UMMA canonical MN-major, no swizzle: 8 x 8 blocks, a row of 8 n-values per k; blocks k_stride / n_stride bytes apart -> float32 [ks, n]."""
+    k = np.arange(ks)[:, None]
+    c = np.arange(n)[None, :]
+    return _halves(buf, (c // 8) * n_stride + (k // 8) * k_stride + (k % 8) * 16 + (c % 8) * 2)
+
+
+def _halves(buf, addr):
+    return from_bits(buf[addr].astype(np.uint16) | (buf[addr + 1].astype(np.uint16) << 8), F16)
 
 
 def put16(buf, addr, halves):
@@ -32,123 +39,112 @@ def put16(buf, addr, halves):
     buf[addr + 1:addr + 16:2] = b >> 8
 
 
-def pf_load8(pool_row, kv_bits, dim0, scale, zero):
-    """8 consecutive dims of one token, de-quantised: fma_T(T(q), scale, zero)."""
+def unpack16(raw, kv_bits, scale, zero):
+    """16 bytes of a token's row -> its dims in order, de-quantised: fma_T(T(q), scale, zero)."""
     if kv_bits == 16:
-        raw = pool_row[dim0 * 2:dim0 * 2 + 16]
         return from_bits(raw[0::2].astype(np.uint16) | (raw[1::2].astype(np.uint16) << 8), F16)
     if kv_bits == 8:
-        q = pool_row[dim0:dim0 + 8].astype(np.float32)
+        q = raw.astype(np.float32)
     else:
-        w = int(pool_row[dim0 // 2:dim0 // 2 + 4].view(np.uint32)[0])
-        n = [(w >> (4 * j)) & 15 for j in range(8)]
-        # cvt_u4x8: registers (n0,n4) (n1,n5) (n2,n6) (n3,n7) -> natural dim order 0..7 by the KV nibble order
-        q = np.array([n[0], n[4], n[1], n[5], n[2], n[6], n[3], n[7]], np.float32)
+        q = []
+        for w in raw.view(np.uint32):
+            n = [(int(w) >> (4 * j)) & 15 for j in range(8)]
+            q += [n[0], n[4], n[1], n[5], n[2], n[6], n[3], n[7]]       # cvt_u4x8 pairs nibbles (j, j + 4); the cache's order undoes it
+        q = np.array(q, np.float32)
     return OA.t_fma(q, np.float32(scale), np.float32(zero), F16)
 
 
-def emulate(pool, block_bytes, tables, cu_q, cu_k, layer_offset, block_len, Hq, Hkv, kv_bits, q_rot, qk_scale, v_pad=0):
-    v_sbo = 128 + v_pad                  # kPfVSbo / kPfVLbo of the kernel (kPfVPad = v_pad)
-    v_lbo = (D // 8) * v_sbo
+def load_tile(pool, kv_bits, block_len, Hkv, h, is_v, table, block_bytes, layer_offset, j, last):
+    """One 128-key operand tile as the seven loader warps fill it."""
+    row_bytes = D * kv_bits // 8
+    units = row_bytes // 16
+    tile = np.full(KEYS * D * 2, 0xA5, np.uint8)
+    for w in range(LOADERS):
+        for i in range(w, KEYS // 8 * (units // 4), LOADERS):
+            for lane in range(32):
+                row, unit = i // (units // 4) * 8 + (lane & 7), i % (units // 4) * 4 + (lane >> 3)
+                key = j * KEYS + row
+                raw, s, z = np.zeros(16, np.uint8), 0.0, 0.0
+                if key <= last:
+                    blk = table[key // block_len] * block_bytes + layer_offset
+                    bt = key % block_len
+                    at = blk + (2 * h + is_v) * block_len * row_bytes + bt * row_bytes + unit * 16
+                    raw = pool[at:at + 16].copy()
+                    if kv_bits != 16:
+                        at = blk + Hkv * 2 * block_len * row_bytes + (2 * h + is_v) * block_len * 4 + bt * 4
+                        s, z = from_bits(pool[at:at + 4].view(np.uint16), F16)
+                x = unpack16(raw, kv_bits, s, z) if key <= last else np.zeros(16 * 8 // kv_bits, np.float32)
+                for c in range(16 // kv_bits):
+                    put16(tile, (unit * (16 // kv_bits) + c) * (KEYS * 16) + row * 16, x[8 * c:8 * c + 8])
+    return tile
+
+
+def emulate(pool, block_bytes, tables, cu_q, cu_k, layer_offset, block_len, Hq, Hkv, kv_bits, q_rot, qk_scale, ctas=0):
     G = Hq // Hkv
     TQ = ROWS // G
-    kRow = D * kv_bits // 8
-    head_data_sz, head_param_sz = block_len * kRow, block_len * 4
-    batch = len(cu_q) - 1
     T = cu_q[-1]
     out = np.zeros((T, Hq * D), np.float32)
-    grid_x = T // TQ + batch
-    for h in range(Hkv):
-        for bx in range(grid_x):
-            x, b = bx, 0
-            while b < batch:
-                nt = (cu_q[b + 1] - cu_q[b] + TQ - 1) // TQ
-                if x < nt:
-                    break
-                x -= nt
-                b += 1
-            if b >= batch:
+    pieces = []                                                         # (sequence, first token, kv-head), places of the list before it
+    place = 0
+    for b in range(len(cu_q) - 1):
+        q_len, hist = cu_q[b + 1] - cu_q[b], cu_k[b + 1] - cu_k[b] - (cu_q[b + 1] - cu_q[b])
+        for q0 in range(0, q_len, 2 * TQ):
+            n = (hist + min(q_len, q0 + 2 * TQ) - 1) // KEYS + 1
+            for h in range(Hkv):
+                pieces.append((b, q0, h, q_len, hist, n, place))
+                place += START + n
+    cuts = [place * c // ctas for c in range(1, ctas)]
+    for b, q0, h, q_len, hist, n, first in pieces:
+        # the piece's key tiles, cut where a range ends
+        edges = sorted({0, n} | {min(n, max(0, c - first - START)) for c in cuts})
+        last = hist + min(q_len, q0 + 2 * TQ) - 1
+        kv = [[load_tile(pool, kv_bits, block_len, Hkv, h, v, tables[b], block_bytes, layer_offset, j, last) for v in (0, 1)] for j in range(n)]
+        K = [read_operand(x[0], KEYS, D, KEYS * 16, 128).astype(np.float64) for x in kv]
+        V = [read_mn_major(x[1], D, KEYS, 128, KEYS * 16).astype(np.float64) for x in kv]
+        for t in range(2):
+            nq = max(0, min(TQ, q_len - q0 - t * TQ))
+            if nq == 0:
                 continue
-            q0 = x * TQ
-            q_len, k_len = cu_q[b + 1] - cu_q[b], cu_k[b + 1] - cu_k[b]
-            hist = k_len - q_len
-            nq = min(TQ, q_len - q0)
-            last_pos = hist + q0 + nq - 1
-            n_tiles = last_pos // KEYS + 1
             r = np.arange(ROWS)
             tq, g = r // G, r % G
             valid = tq < nq
-            pos_q = np.where(valid, hist + q0 + tq, 0x7fffffff)
-            tok = cu_q[b] + q0 + tq
+            pos0 = hist + q0 + t * TQ
+            pos = np.where(valid, pos0 + tq, 0x7fffffff)
+            tok = cu_q[b] + q0 + t * TQ + tq
             q_op = np.zeros(ROWS * D * 2, np.uint8)
-            for row in range(ROWS):
+            for row in np.nonzero(valid)[0]:
                 for c in range(D // 8):
-                    v = q_rot[tok[row], h * G + g[row], c * 8:c * 8 + 8] if valid[row] else np.zeros(8, np.float32)
-                    put16(q_op, (c * ROWS + row) * 16, v)
+                    put16(q_op, (c * ROWS + row) * 16, q_rot[tok[row], h * G + g[row], c * 8:c * 8 + 8])
             Q = read_operand(q_op, ROWS, D, ROWS * 16, 128).astype(np.float64)
-            o = np.zeros((ROWS, D), np.float64)
-            m = np.full(ROWS, -np.inf)
-            l = np.zeros(ROWS)
-            for j in range(n_tiles):
-                key0 = j * KEYS
-                blk = tables[b][key0 // block_len] * block_bytes + layer_offset
-                bt0 = key0 % block_len
-                kd = blk + (h * 2) * head_data_sz + bt0 * kRow
-                vd = kd + head_data_sz
-                kp = blk + Hkv * 2 * head_data_sz + (h * 2) * head_param_sz + bt0 * 4
-                vp = kp + head_param_sz
-                k_op = np.zeros(KEYS * D * 2, np.uint8)
-                v_op = np.zeros((KEYS // 8) * v_lbo, np.uint8)
-
-                def params(base, key):
-                    if kv_bits == 16:
-                        return 0.0, 0.0
-                    pr = from_bits(pool[base + key * 4: base + key * 4 + 4].view(np.uint16), F16)
-                    return pr[0], pr[1]
-
-                for tid in range(128):
-                    key, half = tid & 63, tid >> 6
-                    live = key0 + key <= last_pos
-                    s, z = params(kp, key) if live else (0.0, 0.0)
-                    for cc in range(8):
-                        x8 = pf_load8(pool[kd + key * kRow: kd + (key + 1) * kRow], kv_bits, half * 64 + cc * 8, s, z) \
-                            if live else np.zeros(8, np.float32)
-                        put16(k_op, ((half * 8 + cc) * KEYS + key) * 16, x8)
-                for tid in range(128):
-                    kg, dg = tid >> 4, tid & 15
-                    a = np.zeros((8, 8), np.float32)          # a[jj][dim]: registers a[jj][i>>1] hold dims (2(i>>1), +1)
-                    for jj in range(8):
-                        key = kg * 8 + jj
-                        if key0 + key <= last_pos:
-                            s, z = params(vp, key)
-                            a[jj] = pf_load8(pool[vd + key * kRow: vd + (key + 1) * kRow], kv_bits, dg * 8, s, z)
-                    for i in range(8):
-                        # y[q] = byte_perm(a[2q][i>>1], a[2q+1][i>>1], sel): (key 2q, key 2q+1) of dim i
-                        y = [a[kk][(i >> 1) * 2 + (i & 1)] for kk in range(8)]
-                        put16(v_op, kg * v_lbo + dg * v_sbo + i * 16, y)
-                K = read_operand(k_op, KEYS, D, KEYS * 16, 128).astype(np.float64)       # B of S: N = keys, K = d
-                Vt = read_operand(v_op, D, KEYS, v_lbo, v_sbo).astype(np.float64)       # B of PV: N = d, K = keys
-                S = (Q @ K.T).astype(np.float32)
-                kidx = key0 + np.arange(KEYS)[None, :]
-                Sm = np.where(kidx <= pos_q[:, None], S, -np.inf)
-                m_new = np.maximum(m, Sm.max(1))
-                alpha = np.exp2((m - m_new) * qk_scale)
-                P = np.exp2(Sm.astype(np.float64) * qk_scale - (m_new * qk_scale)[:, None])
-                l = l * alpha + P.sum(1)
-                m = m_new
-                Pt = rn(P.astype(np.float32), F16).astype(np.float64)
-                o = o * alpha[:, None] + Pt @ Vt.T
-            res = rn((o / l[:, None]).astype(np.float32), F16)
-            for row in range(ROWS):
-                if valid[row]:
-                    hq = h * G + g[row]
-                    out[tok[row], hq * D:(hq + 1) * D] = res[row]
+            tiles = (pos0 + nq - 1) // KEYS + 1                         # of this tile of rows
+            M, L, O = np.full(ROWS, -np.inf), np.zeros(ROWS), np.zeros((ROWS, D))
+            for j0, j1 in zip(edges, edges[1:]):
+                m, l, o = np.full(ROWS, -np.inf), np.zeros(ROWS), np.zeros((ROWS, D))
+                for j in range(j0, min(j1, tiles)):
+                    S = (Q @ K[j].T).astype(np.float32)
+                    S = np.where(j * KEYS + np.arange(KEYS)[None, :] <= pos[:, None], S, -np.inf)
+                    m_new = np.maximum(m, S.max(1))
+                    alpha = np.where(m == -np.inf, 0.0, np.exp2((m - np.where(m_new == -np.inf, 0.0, m_new)) * qk_scale))
+                    mc = np.where(m_new == -np.inf, 0.0, m_new)
+                    P = np.exp2((S.astype(np.float64) - mc[:, None]) * qk_scale)
+                    l = l * alpha + P.sum(1)
+                    o = o * alpha[:, None] + rn(P.astype(np.float32), F16).astype(np.float64) @ V[j]
+                    m = m_new
+                # parts in order; a part that holds no key of the row has no maximum
+                with np.errstate(invalid="ignore"):
+                    top = np.maximum(M, m)
+                    a, w = np.where(M == -np.inf, 0.0, np.exp2((M - top) * qk_scale)), np.where(m == -np.inf, 0.0, np.exp2((m - top) * qk_scale))
+                M, L, O = top, L * a + l * w, O * a[:, None] + o * w[:, None]
+            res = rn((O[valid] / L[valid, None]).astype(np.float32), F16)
+            for row, x in zip(np.nonzero(valid)[0], res):
+                hq = h * G + g[row]
+                out[tok[row], hq * D:(hq + 1) * D] = x
     return out
 
 
-@pytest.mark.parametrize("kv_bits,heads,v_pad", [(8, (4, 1), 0), (4, (4, 1), 0), (16, (4, 1), 0), (8, (2, 2), 0),
-                                                 (4, (6, 1), 0), (16, (6, 1), 0), (8, (4, 1), 16), (16, (2, 2), 16)])
-def test_kernel_index_math_reproduces_the_oracle(kv_bits, heads, v_pad):
+@pytest.mark.parametrize("kv_bits,heads,ctas", [(8, (4, 1), 0), (4, (4, 1), 0), (16, (4, 1), 0), (8, (2, 2), 0),
+                                                (4, (6, 1), 0), (16, (6, 1), 0), (8, (4, 1), 16), (16, (2, 2), 16)])
+def test_kernel_index_math_reproduces_the_oracle(kv_bits, heads, ctas):
     Hq, Hkv = heads
     rng = np.random.default_rng(kv_bits * 10 + Hq)
     q_lens, hists = np.array([37, 1, 70]), np.array([0, 70, 30])
@@ -183,7 +179,7 @@ def test_kernel_index_math_reproduces_the_oracle(kv_bits, heads, v_pad):
     cu_k = np.concatenate([[0], np.cumsum(k_lens)]).tolist()
     c = float(np.float32(np.float32(1.4426950408889634) / np.float32(np.sqrt(np.float32(D)))))
     got = emulate(cache.pool.reshape(-1), cache.block_bytes, tables, cu_q, cu_k, cache.layer_offset(layer), block_len, Hq, Hkv,
-                  kv_bits, q_rot, c, v_pad)
+                  kv_bits, q_rot, c, ctas)
     assert np.isfinite(got).all()
     # tiled online softmax vs the oracle's single pass: a few fp16 ulps of an O(1) output
     assert np.abs(got - ref).max() <= 2e-3
