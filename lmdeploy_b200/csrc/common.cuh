@@ -201,6 +201,11 @@ struct TypeOps<half> {
         half2 h = __floats2half2_rn(lo, hi);
         return reinterpret_cast<uint32_t&>(h);
     }
+    // s + lo + hi of a pair, each added exactly and rounded to float
+    static B200_DEVICE void add_pair(float& s, uint32_t pair)
+    {
+        asm("{.reg .b16 lo, hi; mov.b32 {lo, hi}, %1; add.rn.f32.f16 %0, lo, %0; add.rn.f32.f16 %0, hi, %0;}" : "+f"(s) : "r"(pair));
+    }
     static B200_DEVICE uint32_t bcast2(half x)
     {
         half2 h = __half2half2(x);
@@ -267,6 +272,10 @@ struct TypeOps<nv_bfloat16> {
     {
         nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
         return reinterpret_cast<uint32_t&>(h);
+    }
+    static B200_DEVICE void add_pair(float& s, uint32_t pair)
+    {
+        asm("{.reg .b16 lo, hi; mov.b32 {lo, hi}, %1; add.rn.f32.bf16 %0, lo, %0; add.rn.f32.bf16 %0, hi, %0;}" : "+f"(s) : "r"(pair));
     }
     static B200_DEVICE uint32_t bcast2(nv_bfloat16 x)
     {

@@ -11,8 +11,7 @@
 // heads of the group.  Roles of a CTA (one per SM, persistent):
 //   warps 0-3 / 4-7   softmax of tile 0 / 1, thread = row: scores from TMEM, causal mask, base-2 online softmax, P (T) back to
 //                     TMEM as the A operand of P.V, in two halves so that the first half's P.V runs under the second half's
-//                     exponentials; the accumulator stays in TMEM and is rescaled only when a row's maximum has grown by more
-//                     than 2^8 (P <= 256 then, and l is kept on the same reference maximum: the same numbers)
+//                     exponentials; the accumulator stays in TMEM and is rescaled when the maximum of a row of the warp has grown
 //   warp 8            issues every tcgen05.mma: Q.K^T of tile t for the next keys right behind P.V of tile t, so that the tensor
 //                     pipe works on one tile while the other one is in its softmax
 //   warps 9-15        K/V pages -> operand tiles of 128 keys (two-slot rings): T pages by asynchronous copies;
@@ -22,8 +21,12 @@
 // Work: all (unit, kv-head, 128-key tile) triples form one flat list that is cut into equal ranges, one per CTA; a (unit, kv-head)
 // whose keys fall into several ranges leaves fp32 partials (accumulator, row maximum, row sum) that prefill_merge_kernel combines in
 // CTA order (deterministic).  So a chunk of a few tokens over a long history uses every SM, and unequal prompts end together.
+// Precision: weights relative to the true maximum so far, not to one that may lag (the largest weight of a row is then one, which
+// rounding to T leaves alone), and summed as T rounds them (numerator and denominator alike).  Error against 64 bits, prompts of 2048,
+// 1190 and 2048 tokens, f16 / bf16 pages: 3.42e-4 / 2.66e-3; with a maximum that may lag by 2^8 and the sum of the unrounded weights
+// 3.47e-4 / 2.70e-3 (and 178 instead of 181 us); one CTA per 128 rows with a maximum per 64 keys had 3.43e-4 / 2.67e-3.
 // Measured (B200, whole operator; before = one CTA per 128 rows, 64-key tiles, the phases one after another): 2 x 64 tokens over
-// 700-1800 int8 keys, 32 / 8 heads: 160 -> 37 us; prompts of 2048, 1190 and 2048 tokens, f16 pages: 465 -> 192 us (420 TFLOP/s).
+// 700-1800 int8 keys, 32 / 8 heads: 160 -> 37 us; prompts of 2048, 1190 and 2048 tokens, f16 pages: 465 -> 181 us (446 TFLOP/s).
 // A 256 x 128 step takes about 5 k cycles where the tensor pipe needs 2.0 k and the exponentials 2.0 k: T pages wait for their
 // copies (16-byte pieces through the load/store unit move about 17 bytes a cycle), quantised ones for the conversion.
 #pragma once
@@ -39,8 +42,6 @@ constexpr int kPfThreads  = 32 * (8 + 1 + kPfLoaders);  // 16 warps: 128 registe
 constexpr int kPfTile     = kPfKeys * kPfD * 2;  // bytes of a Q, K or V operand tile
 constexpr int kPfStages   = 2;
 constexpr int kPfColS = 0, kPfColO = 256, kPfTmemCols = 512;  // tile t: S / P at t * 128, O at 256 + t * 128
-
-constexpr float kPfLazy   = 8.f;  // log2 of the growth of a row's maximum that forces a rescale
 
 // dynamic shared memory: Q tiles, K and V rings, and the staging tiles of quantised pages
 template<int KVBITS>
@@ -207,7 +208,7 @@ struct PrefillRows: PrefillRowMap<KVBITS> {
     }
 };
 
-// SPLIT: p.partial is there; else whole pieces (a kernel of its own: both walks in one cost registers, 178 -> 190 us on the
+// SPLIT: p.partial is there; else whole pieces (a kernel of its own: both walks in one cost registers, 181 -> 194 us on the
 // prompts above)
 template<class T, int KVBITS, bool SPLIT>
 __global__ void __launch_bounds__(kPfThreads, 1) prefill_attention_kernel(const PrefillParams p)
@@ -496,25 +497,25 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attention_kernel(const 
                 }
                 else {
                     const float m_new = fmaxf(m, mx);
-                    if (__any_sync(0xffffffffu, (m_new - m) * c > kPfLazy)) {
+                    if (__any_sync(0xffffffffu, m_new > m)) {
                         const float alpha = m == -INFINITY ? 0.f : exp2_approx((m - m_new) * c);
                         mbar_wait(smem_u32(&bar_o[t]), pho ^ 1);  // P.V of the previous tile has completed
                         umma::fence_after_sync();
 #pragma unroll 1
-                        for (int ch = 0; ch < kPfD / 16; ++ch) {
-                            uint32_t o[16];
-                            umma::ld_32x32b_x16(to + ch * 16, o);
+                        for (int ch = 0; ch < kPfD / 32; ++ch) {
+                            uint32_t o[32];
+                            umma::ld_32x32b_x32(to + ch * 32, o);
                             umma::wait_ld();
 #pragma unroll
-                            for (int k = 0; k < 16; ++k) o[k] = __float_as_uint(__uint_as_float(o[k]) * alpha);
-                            umma::st_32x32b_x16(to + ch * 16, o);
+                            for (int k = 0; k < 32; ++k) o[k] = __float_as_uint(__uint_as_float(o[k]) * alpha);
+                            umma::st_32x32b_x32(to + ch * 32, o);
                         }
                         l *= alpha;
                         m = m_new;
                     }
                 }
                 const float mc    = m == -INFINITY ? 0.f : m * c;
-                float       l4[4] = {0.f, 0.f, 0.f, 0.f};
+                float       l4[4] = {0.f, 0.f, 0.f, 0.f};  // sums of the weights as T rounds them
 #pragma unroll
                 for (int half = 0; half < 2; ++half) {
                     uint32_t pk[32];
@@ -522,8 +523,8 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attention_kernel(const 
                     for (int k = 0; k < 64; k += 2) {
                         const float p0 = exp2_approx(fmaf(__uint_as_float(v[2 * half + (k >> 5)][k & 31]), c, -mc));
                         const float p1 = exp2_approx(fmaf(__uint_as_float(v[2 * half + (k >> 5)][(k & 31) + 1]), c, -mc));
-                        l4[(k >> 1) & 3] += p0 + p1;
                         pk[k >> 1] = Ops::pack2(p0, p1);  // column c of P holds keys (2c, 2c + 1)
+                        Ops::add_pair(l4[(k >> 1) & 3], pk[k >> 1]);
                     }
                     umma::st_32x32b_x32(ts + half * 32, pk);
                     umma::wait_st();

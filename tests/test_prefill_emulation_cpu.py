@@ -126,9 +126,9 @@ def emulate(pool, block_bytes, tables, cu_q, cu_k, layer_offset, block_len, Hq, 
                     m_new = np.maximum(m, S.max(1))
                     alpha = np.where(m == -np.inf, 0.0, np.exp2((m - np.where(m_new == -np.inf, 0.0, m_new)) * qk_scale))
                     mc = np.where(m_new == -np.inf, 0.0, m_new)
-                    P = np.exp2((S.astype(np.float64) - mc[:, None]) * qk_scale)
-                    l = l * alpha + P.sum(1)
-                    o = o * alpha[:, None] + rn(P.astype(np.float32), F16).astype(np.float64) @ V[j]
+                    P = rn(np.exp2((S.astype(np.float64) - mc[:, None]) * qk_scale).astype(np.float32), F16).astype(np.float64)
+                    l = l * alpha + P.sum(1)                            # of the rounded weights, as the product takes them
+                    o = o * alpha[:, None] + P @ V[j]
                     m = m_new
                 # parts in order; a part that holds no key of the row has no maximum
                 with np.errstate(invalid="ignore"):

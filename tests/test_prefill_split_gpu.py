@@ -38,3 +38,35 @@ def test_cut_work_matches_oracle(lib, kv_bits, dtype, heads, q_lens, hists, more
     # P is rounded to T before P.V and the output is rounded to T (half an ulp each, 2^-12 / 2^-9 relative to values up to 4): as for the whole prompts
     bar = 2e-3 if dtype == F16 else 2e-2
     assert np.isfinite(got).all() and np.abs(got - ref).max() <= bar
+
+
+@pytest.mark.parametrize("dtype", [F16, BF16])
+def test_largest_weight_of_a_row_is_exact(lib, dtype):
+    """A row's largest score stands in its second key tile, 4.5 to 5.4 above the largest of the first: the weight it gets is one, whatever the tile before
+    it had for a maximum, so that the output (that key's value, one, times a normalised weight) is off by its own rounding and little more."""
+    import ctypes as C
+    import torch
+    from lmdeploy_b200 import _lib as L
+    from harness import PagedCase, from_dev_T
+    from oracle import attention as OA
+    from oracle.numerics import rn
+    hist, top = 140, 135
+    case = PagedCase(batch_hist=[hist] * 64, num_heads=4, num_kv_heads=1, kv_bits=16, dtype=dtype, rope=OA.RopeParam(type=OA.ROPE_NULL))
+    u = np.where(np.random.default_rng(1).integers(0, 2, 128) > 0, 1.0, -1.0).astype(np.float32)
+    k, v = np.tile(-4.0 * u, (hist, 1, 1)), np.zeros((hist, 1, 128), np.float32)
+    k[0], k[top], v[top] = 0.0, 0.5 * u, 1.0
+    for table in case.block_tables:
+        OA.process_kv(case.cache, table, case.layer, 0, k, v, case.rope, None, None)
+    gaps = np.linspace(4.5, 5.4, 256)                                       # score of `top`: u.u * 0.5 * size / sqrt(128)
+    size = rn((gaps / (64 / np.sqrt(128.0))).astype(np.float32), dtype)
+    case.qkv[:, :512] = (size[:, None] * u).reshape(64, 512)
+    case.qkv[:, 512:640], case.qkv[:, 640:] = -4.0 * u, 0.0
+    case.upload()
+    ws = torch.zeros(64 * 4 * 256, dtype=torch.uint8, device="cuda")        # no partials: one CTA has both tiles
+    p = case.params(lib, workspace=ws)
+    L.check(lib.b200_prefill_attention(C.byref(p)), "b200_prefill_attention")
+    torch.cuda.synchronize()
+    got = from_dev_T(case.d_out, dtype).reshape(256, 128).astype(np.float64)
+    w = np.exp(-size.astype(np.float64) * 64 / np.sqrt(128.0))              # of key 0; the others' are e^-40
+    half = 2.0 ** -12 if dtype == F16 else 2.0 ** -9                        # half a step between 0.5 and 1
+    assert (np.abs(got - (1 / (1 + w))[:, None]) <= 1.02 * half + 4 * half * w[:, None]).all()
