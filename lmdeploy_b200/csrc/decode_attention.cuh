@@ -396,17 +396,18 @@ struct ConsumerCtx {
 // token's (scale, zero) are applied to the products in fp32:
 //   s_t = scale_t * 2^24 * (code_t . q) + zero_t * sum(q);    P_t = exp2(..),   P'_t = T(P_t * scale_t * kappa)
 //   kappa * O_d = 2^24 * sum_t P'_t code_td + sum_t P'_t * (zero_t / scale_t)
-// The same rounded P' stands in both sums, so its rounding acts on V as before; K and V are no longer rounded to T.  kappa keeps P' in
-// f16's normal range; a tile with a scale outside [kMin, kMax] (0 among them: a constant vector) takes the T-rounded values as the
-// other types do.  Measured (B200, 32 / 8 heads, whole operator): int4, 128 x 4096: 190 -> 171 us; int8, 64 x 2048: 64 -> 59 us (170 and 57 us since, with a faster fix-up);
+// The same rounded P' stands in both sums, so its rounding acts on V as before; K and V are no longer rounded to T.  A warp's 16 keys with
+// a scale outside [kMin, kMax] (0 among them: a constant vector) take the T-rounded values as the other types do: inside, scale * kappa
+// is at least 1, so that P' is nowhere rounded more coarsely than T(P), and at most 2^15, so that it stays finite (P is 1 at most, but
+// for the rounding of the exponent).  Measured (B200, 32 / 8 heads, whole operator): int4, 128 x 4096: 190 -> 171 us; int8, 64 x 2048: 64 -> 59 us (170 and 57 us since, with a faster fix-up);
 // error against 64 bits 5.1e-4 -> 4.4e-4 and 4.9e-4 -> 4.0e-4.
 template<class T, int KVBITS>
 constexpr bool kCodesInMma = std::is_same<T, half>::value && KVBITS != 16;
 template<int KVBITS>
 struct CodeScale {
-    static constexpr float kappa = KVBITS == 8 ? 4096.f : 1024.f;
-    static constexpr float kMin  = KVBITS == 8 ? 1.f / 65536 : 1.f / 16384;
-    static constexpr float kMax  = KVBITS == 8 ? 15.f : 60.f;
+    static constexpr float kappa = KVBITS == 8 ? 65536.f : 16384.f;  // values that span up to 127 (int8: 255 / 2) or 30 (int4: 15 * 2)
+    static constexpr float kMin  = 1.f / kappa;
+    static constexpr float kMax  = 32768.f / kappa;
     // what one unit of accumulator j (pv_dim) stands for
     B200_DEVICE static float unit(int j) { return KVBITS == 8 || !(j & 1) ? 16777216.f : 1048576.f; }
 };
@@ -578,13 +579,13 @@ B200_DEVICE void process_tile(const ConsumerCtx<T, KVBITS>& cx, uint32_t st, boo
     bool     codes = false;  // warp-uniform: the values' codes go into the product as they are
     if constexpr (kCodesInMma<T, KVBITS>) {
         float2 vA = half2_to_float2(lds32(st + Cfg::kOffVP + tokA * 4)), vB = half2_to_float2(lds32(st + Cfg::kOffVP + tokB * 4));
+        using CS = CodeScale<KVBITS>;
         if (maskA) {
-            vA = make_float2(1.f, 0.f);
+            vA = make_float2(CS::kMin, 0.f);
         }
         if (maskB) {
-            vB = make_float2(1.f, 0.f);
+            vB = make_float2(CS::kMin, 0.f);
         }
-        using CS = CodeScale<KVBITS>;
         codes = __all_sync(0xffffffffu, vA.x >= CS::kMin && vA.x <= CS::kMax && vB.x >= CS::kMin && vB.x <= CS::kMax);
         if (codes) {
             const float    kA = vA.x * CS::kappa, kB = vB.x * CS::kappa;
