@@ -395,12 +395,17 @@ struct ConsumerCtx {
 // IS code * 2^-24 (2^-20 four bits up), a subnormal, so a lane costs one permute or mask instead of permute, subtraction and fma; the
 // token's (scale, zero) are applied to the products in fp32:
 //   s_t = scale_t * 2^24 * (code_t . q) + zero_t * sum(q);    P_t = exp2(..),   P'_t = T(P_t * scale_t * kappa)
-//   kappa * O_d = 2^24 * sum_t P'_t code_td + sum_t P'_t * (zero_t / scale_t)
+//   kappa * O_d = 2^24 * sum_t P'_t (code_td - mid) + sum_t P'_t * (zero_t / scale_t + mid)
+// mid is the middle of the codes: the codes enter as they are, and every kRecentre tiles mid * sum P' is taken off the accumulators.  Left
+// in, it makes them a hundred times larger than the output that remains when the zero part is added, and the tensor cores cut a product's
+// bits off at the accumulator's last one (64 sequences of 8192 int8 keys: error against 64 bits 5.3e-4 with T-rounded values, 9.9e-4
+// without this, 4.5e-4 with it).
 // The same rounded P' stands in both sums, so its rounding acts on V as before; K and V are no longer rounded to T.  A warp's 16 keys with
 // a scale outside [kMin, kMax] (0 among them: a constant vector) take the T-rounded values as the other types do: inside, scale * kappa
 // is at least 1, so that P' is nowhere rounded more coarsely than T(P), and at most 2^15, so that it stays finite (P is 1 at most, but
-// for the rounding of the exponent).  Measured (B200, 32 / 8 heads, whole operator): int4, 128 x 4096: 190 -> 171 us; int8, 64 x 2048: 64 -> 59 us (170 and 57 us since, with a faster fix-up);
-// error against 64 bits 5.1e-4 -> 4.4e-4 and 4.9e-4 -> 4.0e-4.
+// for the rounding of the exponent).
+// Measured (B200, 32 / 8 heads, whole operator, T-rounded values -> this): int4, 128 x 4096: 190 -> 174 us, error against 64 bits 5.1e-4 ->
+// 4.3e-4; int8, 64 x 2048: 62 -> 57 us, 4.9e-4 -> 4.0e-4.
 template<class T, int KVBITS>
 constexpr bool kCodesInMma = std::is_same<T, half>::value && KVBITS != 16;
 template<int KVBITS>
@@ -408,6 +413,7 @@ struct CodeScale {
     static constexpr float kappa = KVBITS == 8 ? 65536.f : 16384.f;  // values that span up to 127 (int8: 255 / 2) or 30 (int4: 15 * 2)
     static constexpr float kMin  = 1.f / kappa;
     static constexpr float kMax  = 32768.f / kappa;
+    static constexpr float mid   = KVBITS == 8 ? 128.f : 8.f;
     // what one unit of accumulator j (pv_dim) stands for
     B200_DEVICE static float unit(int j) { return KVBITS == 8 || !(j & 1) ? 16777216.f : 1048576.f; }
 };
@@ -416,11 +422,38 @@ B200_DEVICE float2 half2_to_float2(uint32_t x)
     return __half22float2(reinterpret_cast<const half2&>(x));
 }
 
-// one 64-token tile: this warp's 16 keys.  `st` = shared address of the stage.  Qs: sum over the dims of q (heads 2t, 2t + 1); A: the
-// lane's part of sum P' zero / scale (both kCodesInMma only).
+constexpr int kRecentre = 8;
+
+// kCodesInMma: sums that go with the accumulators of a run of tiles (heads 2t, 2t + 1)
+struct CodeSums {
+    float q[2];  // q's dims
+    float a[2];  // this lane's part of sum P' (zero / scale + mid)
+    float w[2];  // this lane's part of sum P' since mid was last taken off the accumulators
+};
+
+template<int KVBITS>
+B200_DEVICE void recentre(float (&O)[8][4], CodeSums& sums)
+{
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        float w = sums.w[i];
+        w += __shfl_xor_sync(0xffffffffu, w, 4);
+        w += __shfl_xor_sync(0xffffffffu, w, 8);
+        w += __shfl_xor_sync(0xffffffffu, w, 16);
+        sums.w[i] = 0.f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const float f = CodeScale<KVBITS>::mid / CodeScale<KVBITS>::unit(j);
+            O[j][i]       = fmaf(-f, w, O[j][i]);
+            O[j][i + 2]   = fmaf(-f, w, O[j][i + 2]);
+        }
+    }
+}
+
+// one 64-token tile: this warp's 16 keys.  `st` = shared address of the stage.
 template<class T, int KVBITS>
 B200_DEVICE void process_tile(const ConsumerCtx<T, KVBITS>& cx, uint32_t st, bool residue, int k_len, int t0, float c,
-                              const uint32_t (&qf)[8][2], float (&O)[8][4], float (&M)[2], float (&L)[2], const float (&Qs)[2], float (&A)[2])
+                              const uint32_t (&qf)[8][2], float (&O)[8][4], float (&M)[2], float (&L)[2], CodeSums& sums)
 {
     using Ops = TypeOps<T>;
     using Cfg = TileCfg<KVBITS>;
@@ -462,10 +495,10 @@ B200_DEVICE void process_tile(const ConsumerCtx<T, KVBITS>& cx, uint32_t st, boo
             for (int i = 0; i < 4; ++i) S[i] = fmaf(S4[i], 0.0625f, S[i]);
         }
         const float sA = zA.x * 16777216.f, sB = zB.x * 16777216.f;
-        S[0] = fmaf(sA, S[0], zA.y * Qs[0]);
-        S[1] = fmaf(sA, S[1], zA.y * Qs[1]);
-        S[2] = fmaf(sB, S[2], zB.y * Qs[0]);
-        S[3] = fmaf(sB, S[3], zB.y * Qs[1]);
+        S[0] = fmaf(sA, S[0], zA.y * sums.q[0]);
+        S[1] = fmaf(sA, S[1], zA.y * sums.q[1]);
+        S[2] = fmaf(sB, S[2], zB.y * sums.q[0]);
+        S[3] = fmaf(sB, S[3], zB.y * sums.q[1]);
     }
     else if constexpr (KVBITS == 8) {
         const uint32_t pA  = lds32(st + Cfg::kOffKP + tokA * 4);
@@ -553,8 +586,8 @@ B200_DEVICE void process_tile(const ConsumerCtx<T, KVBITS>& cx, uint32_t st, boo
         L[0] *= r0;
         L[1] *= r1;
         if constexpr (kCodesInMma<T, KVBITS>) {
-            A[0] *= r0;
-            A[1] *= r1;
+            sums.a[0] *= r0, sums.w[0] *= r0;
+            sums.a[1] *= r1, sums.w[1] *= r1;
         }
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
@@ -590,10 +623,12 @@ B200_DEVICE void process_tile(const ConsumerCtx<T, KVBITS>& cx, uint32_t st, boo
         if (codes) {
             const float    kA = vA.x * CS::kappa, kB = vB.x * CS::kappa;
             const uint32_t wA = Ops::pack2(P[0] * kA, P[1] * kA), wB = Ops::pack2(P[2] * kB, P[3] * kB);
-            const float    rA = __fdividef(vA.y, vA.x), rB = __fdividef(vB.y, vB.x);
+            const float    rA = __fdividef(vA.y, vA.x) + CS::mid, rB = __fdividef(vB.y, vB.x) + CS::mid;
             const float2   fA = half2_to_float2(wA), fB = half2_to_float2(wB);
-            A[0] = fmaf(fA.x, rA, fmaf(fB.x, rB, A[0]));
-            A[1] = fmaf(fA.y, rA, fmaf(fB.y, rB, A[1]));
+            sums.a[0] = fmaf(fA.x, rA, fmaf(fB.x, rB, sums.a[0]));
+            sums.a[1] = fmaf(fA.y, rA, fmaf(fB.y, rB, sums.a[1]));
+            sums.w[0] += fA.x + fB.x;
+            sums.w[1] += fA.y + fB.y;
             pf[0] = transpose_8x8_b16(wA);
             pf[1] = transpose_8x8_b16(wB);
         }
@@ -1099,7 +1134,7 @@ __global__ void __launch_bounds__(kThreads, min_ctas_per_sm<KVBITS>()) decode_at
     uint32_t qf[8][2];  // Q as B-operand fragments, one per k-step
     float    O[8][4];   // O^T accumulators: m-tile j -> {(slot g,head 2t),(g,2t+1),(g+8,2t),(g+8,2t+1)}
     float    M[2], L[2];
-    float    Qs[2] = {0.f, 0.f}, A[2] = {0.f, 0.f};  // kCodesInMma: sums over q's dims, sum P' zero / scale
+    CodeSums sums{};
 
     const float c = p.qk_scale;
 
@@ -1160,7 +1195,7 @@ __global__ void __launch_bounds__(kThreads, min_ctas_per_sm<KVBITS>()) decode_at
             M[0] = M[1] = -INFINITY;
             L[0] = L[1] = 0.f;
             if constexpr (kCodesInMma<T, KVBITS>) {
-                A[0] = A[1] = 0.f;
+                sums.a[0] = sums.a[1] = sums.w[0] = sums.w[1] = 0.f;
                 float q = 0.f;  // head g: this lane's 32 dims, then all 128
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
@@ -1169,19 +1204,28 @@ __global__ void __launch_bounds__(kThreads, min_ctas_per_sm<KVBITS>()) decode_at
                 }
                 q += __shfl_xor_sync(0xffffffffu, q, 1);
                 q += __shfl_xor_sync(0xffffffffu, q, 2);
-                Qs[0] = __shfl_sync(0xffffffffu, q, 8 * t);
-                Qs[1] = __shfl_sync(0xffffffffu, q, 8 * t + 4);
+                sums.q[0] = __shfl_sync(0xffffffffu, q, 8 * t);
+                sums.q[1] = __shfl_sync(0xffffffffu, q, 8 * t + 4);
             }
         }
         // The tile that holds the new token (position k_len - 1, always the sequence's last tile) is peeled out of the loop:
         // the out-of-line prologue call must not sit inside the loop (the ABI would pin the loop state in local memory).
         const bool peel  = (p.fused & 1) && first_tile + ntile == it.tiles;
         const int  nloop = ntile - (peel ? 1 : 0);
+        // before a tile, not behind it: the peeled form takes the same steps
+        auto recentre_at = [&](int tt) {
+            if constexpr (kCodesInMma<T, KVBITS>) {
+                if (tt > 0 && tt % kRecentre == 0) {
+                    recentre<KVBITS>(O, sums);
+                }
+            }
+        };
         for (int tt = 0; tt < nloop; ++tt) {
             const int  t0      = (first_tile + tt) * kTile;
             const bool residue = t0 + kTile > k_len;
+            recentre_at(tt);
             mbar_wait(full0 + 8 * s, ph);
-            process_tile<T, KVBITS>(cx, stage0 + s * (uint32_t)Cfg::kStageBytes, residue, k_len, t0, c, qf, O, M, L, Qs, A);
+            process_tile<T, KVBITS>(cx, stage0 + s * (uint32_t)Cfg::kStageBytes, residue, k_len, t0, c, qf, O, M, L, sums);
             __syncwarp();
             if (lane == 0) {
                 mbar_arrive(empty0 + 8 * s);
@@ -1193,6 +1237,7 @@ __global__ void __launch_bounds__(kThreads, min_ctas_per_sm<KVBITS>()) decode_at
         }
         if (peel) {
             const int t0 = (it.tiles - 1) * kTile;
+            recentre_at(nloop);
             mbar_wait(full0 + 8 * s, ph);
             // The new token's slot belongs to exactly one consumer warp (slot_token: token & 15 = 4 * warp + i): that warp runs
             // the prologue for this (sequence, kv-head) -- bias, RoPE(k), quantise, store into the page for later steps -- and
@@ -1202,7 +1247,7 @@ __global__ void __launch_bounds__(kThreads, min_ctas_per_sm<KVBITS>()) decode_at
                 new_token_kv<T, KVBITS>(p, it.b, it.h, k_len - 1, pos, lane, stage0 + s * (uint32_t)Cfg::kStageBytes);
                 __syncwarp();
             }
-            process_tile<T, KVBITS>(cx, stage0 + s * (uint32_t)Cfg::kStageBytes, true, k_len, t0, c, qf, O, M, L, Qs, A);
+            process_tile<T, KVBITS>(cx, stage0 + s * (uint32_t)Cfg::kStageBytes, true, k_len, t0, c, qf, O, M, L, sums);
             __syncwarp();
             if (lane == 0) {
                 mbar_arrive(empty0 + 8 * s);
@@ -1215,20 +1260,24 @@ __global__ void __launch_bounds__(kThreads, min_ctas_per_sm<KVBITS>()) decode_at
         const bool last_tile = first_tile + ntile == it.tiles;
 
         // ---------------- segment end: merge the 4 consumer warps, write final or partial ----------------
+        if constexpr (kCodesInMma<T, KVBITS>) {
+            recentre<KVBITS>(O, sums);
+        }
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
             L[q] += __shfl_xor_sync(0xffffffffu, L[q], 4);
             L[q] += __shfl_xor_sync(0xffffffffu, L[q], 8);
             L[q] += __shfl_xor_sync(0xffffffffu, L[q], 16);
             if constexpr (kCodesInMma<T, KVBITS>) {
-                A[q] += __shfl_xor_sync(0xffffffffu, A[q], 4);
-                A[q] += __shfl_xor_sync(0xffffffffu, A[q], 8);
-                A[q] += __shfl_xor_sync(0xffffffffu, A[q], 16);
+                float A = sums.a[q];
+                A += __shfl_xor_sync(0xffffffffu, A, 4);
+                A += __shfl_xor_sync(0xffffffffu, A, 8);
+                A += __shfl_xor_sync(0xffffffffu, A, 16);
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
                     const float u = CodeScale<KVBITS>::unit(j);
-                    O[j][q]       = fmaf(O[j][q], u, A[q]) * (1.f / CodeScale<KVBITS>::kappa);
-                    O[j][q + 2]   = fmaf(O[j][q + 2], u, A[q]) * (1.f / CodeScale<KVBITS>::kappa);
+                    O[j][q]       = fmaf(O[j][q], u, A) * (1.f / CodeScale<KVBITS>::kappa);
+                    O[j][q + 2]   = fmaf(O[j][q + 2], u, A) * (1.f / CodeScale<KVBITS>::kappa);
                 }
             }
         }

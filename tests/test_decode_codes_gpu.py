@@ -148,3 +148,29 @@ def test_long_tail_of_small_weights_over_narrow_values(kv_bits, gap, monkeypatch
     bar = U * np.abs(ref) + 2 * U * tail + 149 * 16 * 2.0 ** -25 * 2 + 2.0 ** -18
     err = np.abs(got - ref)
     assert (err <= bar).all(), float((err / bar).max())
+
+
+@pytest.mark.parametrize("kv_bits", [8, 4])
+def test_long_even_contexts_keep_their_bits(kv_bits, lib):
+    """16 384 keys of like weight: the output is a hundredth of a value, so that sums which carried the values' offset would lose it."""
+    import torch
+    case = PagedCase(batch_hist=[HIST], num_heads=4, num_kv_heads=1, kv_bits=kv_bits, seed=9, rope=OA.RopeParam(type=OA.ROPE_NULL))
+    rng = np.random.default_rng(10)
+    qkv = rn(rng.standard_normal((BATCH, 6 * 128)).astype(np.float32), F16)
+    got = torch.from_numpy(_shared_pages(case, lib, qkv).astype(np.float64))
+    keep, OA.kv_dequant = OA.kv_dequant, _dequant64
+    try:
+        K, V = (torch.from_numpy(x) for x in case.cache.read_tokens(case.block_tables[0], case.layer, 0, HIST))
+        new = [OA.PagedKvCache(BATCH, 1, case.layout, F16) for _ in range(1)][0]
+        for b in range(BATCH):
+            new.write_token(b, 0, 0, 0, qkv[b, 512:640], qkv[b, 640:])
+        nk, nv = (torch.from_numpy(np.stack(x)) for x in zip(*[[y[0] for y in new.read_tokens([b], 0, 0, 1)] for b in range(BATCH)]))
+    finally:
+        OA.kv_dequant = keep
+    q = torch.from_numpy(qkv[:, :512].astype(np.float64)).view(BATCH, 4, 128)
+    s = torch.cat([q @ K.T, (q * nk[:, None]).sum(-1, keepdim=True)], -1) / np.sqrt(128.0)
+    p = s.softmax(-1)
+    ref = p[..., :HIST] @ V + p[..., HIST:] * nv[:, None]
+    # at most four independent roundings to f16 -- keys (as an error of the weights of up to one score's size), weights, values, result -- each up to U,
+    # evenly spread: U / sqrt(3) of the 2-norm
+    assert float((got - ref).norm() / ref.norm()) <= U * (4 / 3) ** 0.5
