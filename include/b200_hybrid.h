@@ -221,6 +221,8 @@ typedef struct b200h_window_args {
     int out_norm;
     float lambda;            /* maps 2: factor on the second map's weights */
     float out_scale;         /* factor on the output (1: none) */
+    int sequences;           /* how many sequences the n rows come from, as a hint to b200h_window_attention (it chooses between two forms of the
+                              * same result); 0: not known, taken for n sequences of one row */
     int64_t ld_y;            /* row stride of y; 0: heads * vdim */
 } b200h_window_args;
 /* Bias, norm of query and key, cache store of key and value (fills qn). */

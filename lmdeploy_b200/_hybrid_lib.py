@@ -51,7 +51,8 @@ class WindowArgs(C.Structure):
         ("tok_seq", C.c_void_p), ("tok_pos", C.c_void_p), ("block_ptrs", C.c_void_p), ("cu_blocks", C.c_void_p),
         ("layer_off", C.c_int64), ("v_off", C.c_int64), ("dtype", C.c_int), ("stream", C.c_void_p), ("sink", C.c_void_p),
         ("chunk", C.c_int), ("talk_scores", C.c_int), ("gate_heads", C.c_int), ("q_temp_coef", C.c_float), ("q_temp_every", C.c_double),
-        ("maps", C.c_int), ("keep_first", C.c_int), ("out_norm", C.c_int), ("lambda_", C.c_float), ("out_scale", C.c_float), ("ld_y", C.c_int64),
+        ("maps", C.c_int), ("keep_first", C.c_int), ("out_norm", C.c_int), ("lambda_", C.c_float), ("out_scale", C.c_float),
+        ("sequences", C.c_int), ("ld_y", C.c_int64),
     ]
 
     def __init__(self, **kw):

@@ -1461,12 +1461,10 @@ static int launch_window_attention(const b200h_window_args* a, WindowGeom g, cud
 }
 
 // ------------------------------------------------------------------------------------------------ the one-pass form (flash_attention.cuh)
-// Whether a call's rows and layout suit flash_attention_kernel.  The line lies between steps of single tokens, whose rows fill a
-// 128-row tile with one token (64 sequences at 1000 keys, 16 / 8 heads of 128, projection included: 142 us by the two passes, which cut
-// a row's keys between blocks, 221 us here) and prompt portions (100 + 100 rows behind 300: 132 and 57 us; 300 rows: 109 and 46 us).
+// Whether flash_attention_kernel can take a call's layout, and whether it should.
 constexpr int kFaMinRows = 96;
 
-static bool flash_attention_takes(const b200h_window_args* a)
+static bool flash_attention_fits(const b200h_window_args* a)
 {
     const int maps = a->maps > 1 ? a->maps : 1, rep = a->heads / a->kv_heads;
     const bool shape = (maps == 1 && a->dim == 128 && a->vdim == 128) || (maps == 1 && a->dim == 64 && a->vdim == 64) || (maps == 2 && a->dim == 64 && a->vdim == 128);
@@ -1475,8 +1473,30 @@ static bool flash_attention_takes(const b200h_window_args* a)
     return a->dtype == B200H_BF16 && shape && rep <= 128 && !a->talk && a->softcap <= 0.f && !a->r1 && a->block_len % 64 == 0 && a->layer_off % 16 == 0 &&
            a->v_off % 16 == 0 && ld_y % 8 == 0 && aligned(a->y) && aligned(a->qn) && aligned(a->o_part) && aligned(a->scores) &&
            (!a->gate || a->gate_heads || (a->ld_gate % 8 == 0 && aligned(a->gate))) &&
-           (int64_t)a->heads * maps * a->score_ld >= 32 &&              // room for the plan: 9 n + 7 ints
-           a->n >= kFaMinRows;
+           (int64_t)a->heads * maps * a->score_ld >= 32;                // room for the plan: 9 n + 7 ints
+}
+
+// The one-pass kernel gives every sequence units of its own, and a 128-row tile costs the same with one token in it as when it is full; a
+// unit's keys are not cut between SMs.  The two passes pay per row and cut a row's keys.  Both costs in microseconds per 128 keys, fitted
+// to 1 - 16 key/value heads of 1 - 16 heads each and 96 - 4096 rows of 1 - 4096 per sequence on a B200 (148 SMs): one pass 0.038 per
+// piece, at least 3.7 or, where a unit has both tiles, 5.0, and 10 in all for its plan; two passes, per row, 0.018 per key/value head or
+// 0.009 per head, whichever is more, 1.55 / 2.1 times that under 8 / 4 key/value heads (most of their second kernel's threads idle), and 8
+// in all where they do not cut the keys.  No measured shape is slower than by the two passes.
+// Whole layer, two passes -> one pass: 128 sequences of one row at 1000 keys, 16 / 8 heads: 210 -> 357 us (two passes are taken), 32 / 2
+// heads: 482 -> 121 us; 128 of two rows, 16 / 8 heads: 348 -> 361 us, of three: 523 -> 363 us; one of 128 rows: 210 -> 78 us; 100 rows
+// behind 8000 keys, 2 / 1 heads: 278 -> 349 us, 16 / 8 heads: 906 -> 357 us; a prompt of 96 rows, 4 / 1 heads: 29 -> 33 us.
+static bool flash_attention_pays(const b200h_window_args* a)
+{
+    const int maps = a->maps > 1 ? a->maps : 1, rep = a->heads / a->kv_heads, unit = (maps == 2 ? 1 : 2) * (128 / rep);
+    const int sequences = a->sequences > 0 && a->sequences < a->n ? a->sequences : a->n;
+    auto larger = [](double x, double y) { return x > y ? x : y; };
+    const double rows = (double)a->n / sequences, ld = (double)a->score_ld;
+    const double tiles = larger(1.0, (ld - (rows < ld ? rows : ld) / 2 - 128) / 128);      // a row's keys, from the longest row's, rounded up to 256
+    const double pieces = (sequences + (a->n - sequences) / unit) * (double)a->kv_heads;
+    const double one = 10.0 + tiles * larger(0.038 * pieces, maps == 1 && 2 * rows <= unit ? 3.7 : 5.0);
+    const double two = tiles * a->n * larger(0.018 * a->kv_heads, 0.009 * a->heads) * (a->kv_heads >= 8 ? 1.0 : a->kv_heads >= 4 ? 1.55 : 2.1) +
+                       (a->splits == 1 ? 8.0 : 0.0);
+    return a->n >= kFaMinRows && one < two;
 }
 
 template <int D, int MAPS, int V>
@@ -1519,7 +1539,7 @@ B200H_API int b200h_window_attention(const b200h_window_args* a)
     if (!a->ml || !a->o_part || !a->y || a->splits < 1 || a->splits > 65535 || a->kv_heads > 32767 || a->heads > 65535 || (a->out_norm && a->vdim > 8192) || (a->r1 && !a->r2))
         return fail(B200H_ERR_INVALID_ARG, "window_attention: bad arguments");
     if (a->n == 0) return 0;
-    if (flash_attention_takes(a)) {
+    if (flash_attention_fits(a) && flash_attention_pays(a)) {
         if (const int rc = launch_flash_attention(a, (cudaStream_t)a->stream)) return rc;
         return launched("window_attention");
     }

@@ -272,7 +272,8 @@ class TurboMind:
             return self.model.step(n=n, batch=B, tokens=d_ctl[:n], tok_seq=d_ctl[n:2 * n], tok_pos=d_ctl[2 * n:3 * n],
                                    cu_q=d_ctl[o:o + B + 1], cu_blocks=d_ctl[o + B + 1:o + 2 * B + 2],
                                    seq_slot=d_ctl[o + 2 * B + 2:o + 3 * B + 2], block_ptrs=d_ptrs, state=self.state,
-                                   rows=d_ctl[o + 3 * B + 2:], n_rows=r, max_pos=max_pos, trace=trace)
+                                   rows=d_ctl[o + 3 * B + 2:], n_rows=r, max_pos=max_pos, trace=trace,
+                                   seq_rows=[cu_q[i + 1] - cu_q[i] for i in range(B)])
 
         # A step of single decoded tokens is shape-static given its batch size and the attention's key ranges: every array lives
         # in a fixed device buffer, so its launches are replayed from a CUDA graph, captured the second time the key is seen

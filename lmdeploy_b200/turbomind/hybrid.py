@@ -22,6 +22,7 @@ design wants in 32 bits (residual stream and its history, norms, rotary angles, 
 is float in every kernel whatever the projection type is."""
 import contextlib
 import ctypes as C
+import itertools
 
 import torch
 
@@ -650,10 +651,10 @@ class HybridModel:
         return torch.mm(x, w.t())
 
     def step(self, *, n, batch, tokens, tok_seq, tok_pos, cu_q, seq_slot, block_ptrs, cu_blocks, state: StatePool, rows, n_rows,
-             max_pos, trace=None):
+             max_pos, trace=None, seq_rows=None):
         """One mixed step.  Device tensors: tokens / tok_seq / tok_pos int32 [n]; cu_q, cu_blocks int32 [batch + 1]; seq_slot
         int32 [batch]; block_ptrs int64 (page addresses); rows int32 [n_rows] = the rows whose logits are wanted; max_pos (host
-        int) = the largest position of the step.
+        int) = the largest position of the step; seq_rows (host list, optional) = how many of the n rows each sequence has.
         Returns float logits [n_rows, vocab].  trace: a list that receives a copy of the stream after every layer."""
         s, lib, w, dev, T, dt = self.spec, self.lib, self.w, self.device, self.T, self.dt
         W, eps, groups = s.width, s.norm_eps, s.norm_groups
@@ -663,25 +664,25 @@ class HybridModel:
         if s.block == "streams":
             return self._step_streams(n=n, batch=batch, tokens=tokens, tok_seq=tok_seq, tok_pos=tok_pos, cu_q=cu_q, seq_slot=seq_slot,
                                       block_ptrs=block_ptrs, cu_blocks=cu_blocks, state=state, rows=rows, n_rows=n_rows, max_pos=max_pos,
-                                      trace=trace)
+                                      trace=trace, seq_rows=seq_rows)
         if s.block == "sandwich":
             return self._step_sandwich(n=n, batch=batch, tokens=tokens, tok_seq=tok_seq, tok_pos=tok_pos, cu_q=cu_q, seq_slot=seq_slot,
                                        block_ptrs=block_ptrs, cu_blocks=cu_blocks, state=state, rows=rows, n_rows=n_rows, max_pos=max_pos,
-                                       trace=trace)
+                                       trace=trace, seq_rows=seq_rows)
         if s.block == "shared_norm":
             return self._step_shared_norm(n=n, batch=batch, tokens=tokens, tok_seq=tok_seq, tok_pos=tok_pos, cu_q=cu_q, seq_slot=seq_slot,
                                           block_ptrs=block_ptrs, cu_blocks=cu_blocks, state=state, rows=rows, n_rows=n_rows,
-                                          max_pos=max_pos, trace=trace)
+                                          max_pos=max_pos, trace=trace, seq_rows=seq_rows)
         if s.block == "parallel":
             return self._step_parallel(n=n, batch=batch, tokens=tokens, tok_seq=tok_seq, tok_pos=tok_pos, cu_q=cu_q, seq_slot=seq_slot,
                                        block_ptrs=block_ptrs, cu_blocks=cu_blocks, state=state, rows=rows, n_rows=n_rows, max_pos=max_pos,
-                                       trace=trace)
+                                       trace=trace, seq_rows=seq_rows)
         if s.block == "pre_norm":
             return self._step_pre_norm(n=n, batch=batch, tokens=tokens, tok_seq=tok_seq, tok_pos=tok_pos, cu_q=cu_q, seq_slot=seq_slot,
                                        block_ptrs=block_ptrs, cu_blocks=cu_blocks, state=state, rows=rows, n_rows=n_rows, max_pos=max_pos,
-                                       trace=trace)
+                                       trace=trace, seq_rows=seq_rows)
         c = StepArrays(n=n, batch=batch, tok_seq=tok_seq, tok_pos=tok_pos, cu_q=cu_q, seq_slot=seq_slot, block_ptrs=block_ptrs,
-                       cu_blocks=cu_blocks, state=state, max_pos=max_pos)
+                       cu_blocks=cu_blocks, state=state, max_pos=max_pos, seq_rows=seq_rows)
         f32 = dict(dtype=torch.float32, device=dev)
         hist = torch.empty(len(s.layers) + 1, n, W, **f32)
         x = torch.empty(n, W, **f32)
@@ -717,13 +718,13 @@ class HybridModel:
             return self._logits(xn)
 
     def _step_pre_norm(self, *, n, batch, tokens, tok_seq, tok_pos, cu_q, seq_slot, block_ptrs, cu_blocks, state, rows, n_rows, max_pos,
-                       trace=None):
+                       trace=None, seq_rows=None):
         """The step of pre-norm blocks: x <- x + mixer(conv(norm1(x))), x <- x + ff(conv(norm2(x))) per run.  A sublayer's output
         joins the float stream inside the kernel that norms the stream for the next reader (residual add + norm in one pass)."""
         s, lib, w, dev, T, dt = self.spec, self.lib, self.w, self.device, self.T, self.dt
         W, eps, st = s.width, s.norm_eps, self._stream()
         c = StepArrays(n=n, batch=batch, tok_seq=tok_seq, tok_pos=tok_pos, cu_q=cu_q, seq_slot=seq_slot, block_ptrs=block_ptrs,
-                       cu_blocks=cu_blocks, state=state, max_pos=max_pos)
+                       cu_blocks=cu_blocks, state=state, max_pos=max_pos, seq_rows=seq_rows)
         x = torch.empty(n, W, dtype=torch.float32, device=dev)
         with self.timed("embed"):
             H.check(lib.b200h_embed(tokens.data_ptr(), w["embed"].data_ptr(), s.embedding_scale, x.data_ptr(), n, W, dt, st), "embed")
@@ -756,14 +757,14 @@ class HybridModel:
             return self._logits(xn)
 
     def _step_parallel(self, *, n, batch, tokens, tok_seq, tok_pos, cu_q, seq_slot, block_ptrs, cu_blocks, state, rows, n_rows, max_pos,
-                       trace=None):
+                       trace=None, seq_rows=None):
         """The step of parallel blocks: x <- x + mult * (mixer(n1(x)) + ff(n2(x))) per run, both sublayers reading the same stream.
         One kernel per run takes the previous run's two outputs into the float stream (and, before a pass of looped layers, the
         embedding output and the pass's vector) and emits both normed inputs of this run."""
         s, lib, w, dev, T, dt = self.spec, self.lib, self.w, self.device, self.T, self.dt
         W, eps, st = s.width, s.norm_eps, self._stream()
         c = StepArrays(n=n, batch=batch, tok_seq=tok_seq, tok_pos=tok_pos, cu_q=cu_q, seq_slot=seq_slot, block_ptrs=block_ptrs,
-                       cu_blocks=cu_blocks, state=state, max_pos=max_pos)
+                       cu_blocks=cu_blocks, state=state, max_pos=max_pos, seq_rows=seq_rows)
         x = torch.empty(n, W, dtype=torch.float32, device=dev)
         with self.timed("embed"):
             H.check(lib.b200h_embed(tokens.data_ptr(), w["embed"].data_ptr(), s.embedding_scale, x.data_ptr(), n, W, dt, st), "embed")
@@ -812,14 +813,14 @@ class HybridModel:
             return self._logits(xn)
 
     def _step_shared_norm(self, *, n, batch, tokens, tok_seq, tok_pos, cu_q, seq_slot, block_ptrs, cu_blocks, state, rows, n_rows, max_pos,
-                          trace=None):
+                          trace=None, seq_rows=None):
         """The step of shared-norm blocks: h = n(x), x <- x + mixer(shift(h)) + ff(h) per run.  One kernel per run takes the previous
         run's outputs (the two sides of a paired mixer, each normed over the width, and the feed-forward's) into the float stream and
         emits this run's normed rows; one kernel shifts them (and forms the recurrence's blends) against the previous token's."""
         s, lib, w, dev, T, dt = self.spec, self.lib, self.w, self.device, self.T, self.dt
         W, eps, st = s.width, s.norm_eps, self._stream()
         c = StepArrays(n=n, batch=batch, tok_seq=tok_seq, tok_pos=tok_pos, cu_q=cu_q, seq_slot=seq_slot, block_ptrs=block_ptrs,
-                       cu_blocks=cu_blocks, state=state, max_pos=max_pos)
+                       cu_blocks=cu_blocks, state=state, max_pos=max_pos, seq_rows=seq_rows)
         stride = state.storage.stride(0)
         x = torch.empty(n, W, dtype=torch.float32, device=dev)
         with self.timed("embed"):
@@ -885,14 +886,14 @@ class HybridModel:
             return self._logits(xn)
 
     def _step_sandwich(self, *, n, batch, tokens, tok_seq, tok_pos, cu_q, seq_slot, block_ptrs, cu_blocks, state, rows, n_rows, max_pos,
-                       trace=None):
+                       trace=None, seq_rows=None):
         """The step of sandwich blocks: x <- x + n1b(mixer(n1(x))), x <- x + n2b(ff(n2(x))) per run.  One kernel per sublayer takes the
         previous sublayer's output (the two sides of a paired mixer, one row, or the chosen experts' parts beside the shared one's),
         norms it, adds it to the float stream and emits the next sublayer's normed input."""
         s, lib, w, dev, T, dt = self.spec, self.lib, self.w, self.device, self.T, self.dt
         W, eps, st = s.width, s.norm_eps, self._stream()
         c = StepArrays(n=n, batch=batch, tok_seq=tok_seq, tok_pos=tok_pos, cu_q=cu_q, seq_slot=seq_slot, block_ptrs=block_ptrs,
-                       cu_blocks=cu_blocks, state=state, max_pos=max_pos)
+                       cu_blocks=cu_blocks, state=state, max_pos=max_pos, seq_rows=seq_rows)
         x = torch.empty(n, W, dtype=torch.float32, device=dev)
         with self.timed("embed"):
             H.check(lib.b200h_embed(tokens.data_ptr(), w["embed"].data_ptr(), s.embedding_scale, x.data_ptr(), n, W, dt, st), "embed")
@@ -954,14 +955,14 @@ class HybridModel:
             return self._logits(xn)
 
     def _step_streams(self, *, n, batch, tokens, tok_seq, tok_pos, cu_q, seq_slot, block_ptrs, cu_blocks, state, rows, n_rows, max_pos,
-                      trace=None):
+                      trace=None, seq_rows=None):
         """The step of stream blocks: the residual is `streams` copies x_s; per sublayer u = sum_s in[s] x_s, y = ls * sublayer(n(u)),
         x_t <- sum_s mix[s, t] x_s + out[t] * y, all streams at once.  One kernel joins a sublayer's output into the streams and emits
         the next sublayer's normed input; the last join runs only over the rows whose logits are wanted."""
         s, lib, w, dev, T, dt = self.spec, self.lib, self.w, self.device, self.T, self.dt
         W, S, eps, st = s.width, s.streams, s.norm_eps, self._stream()
         c = StepArrays(n=n, batch=batch, tok_seq=tok_seq, tok_pos=tok_pos, cu_q=cu_q, seq_slot=seq_slot, block_ptrs=block_ptrs,
-                       cu_blocks=cu_blocks, state=state, max_pos=max_pos)
+                       cu_blocks=cu_blocks, state=state, max_pos=max_pos, seq_rows=seq_rows)
         x = torch.empty(n, S, W, dtype=torch.float32, device=dev)
         h = torch.empty(n, W, dtype=T, device=dev)
         subs = [(r, i, q) for r, (i, _) in enumerate(self.runs) for q in ((1, 2) if s.layers[i].mlp is not None else (1,))]
@@ -1224,7 +1225,6 @@ class HybridModel:
         a = H.WindowArgs()
         a.n, a.heads, a.kv_heads, a.dim, a.vdim, a.block_len, a.window = n, m.heads, m.kv_heads, m.dim, m.vdim, self.block_len, m.window
         a.chunk, a.talk_scores, a.gate_heads = m.chunk, int(m.talk_scores), int(m.gate_per_head)
-        a.splits = self.window_splits(n, m.span, c.max_pos)
         a.scale, a.softcap, a.eps = m.scale, m.softcap, self.spec.norm_eps
         a.maps, a.keep_first, a.out_scale = m.maps, m.keep_first, scale
         if m.maps == 2:
@@ -1263,30 +1263,55 @@ class HybridModel:
         self._window_attend(a, m, c, qn, y, "chunked attention" if m.chunk else "windowed attention")
         return y
 
+    def _attention_runs(self, a, c):
+        """Rows that go to b200h_window_attention together: (first row, rows, sequences to tell it).  The whole step, except where a step mixes many
+        sequences of one row with a prompt portion in a layer that the one-pass kernel can take: the two forms' costs of a single row (microseconds
+        per 128 keys, beside flash_attention_pays in the library) say how much the single rows cost there that they would not cost by themselves; from
+        60 us on they go apart.  16 / 8 heads: 64 sequences at 4000 keys beside a prompt of 200 rows take 529 us by the two passes, 736 us by one,
+        390 us apart; 16 at 1000 keys beside 200 rows 235, 72 and 112 us."""
+        counts = getattr(c, "seq_rows", None)
+        if not counts or a.dtype != H.BF16 or a.softcap > 0 or a.talk or a.r1 or (a.maps, a.dim, a.vdim) not in ((1, 128, 128), (1, 64, 64), (2, 64, 128)):
+            return [(0, c.n, c.batch)]
+        runs, at = [], 0
+        for single, group in itertools.groupby(counts, lambda rows: rows <= 1):
+            group = list(group)
+            runs.append((at, sum(group), len(group)))
+            at += sum(group)
+        singles = sum(rows <= 1 for rows in counts)
+        alone = max(0.018 * a.kv_heads, 0.009 * a.heads) * (1.0 if a.kv_heads >= 8 else 1.55 if a.kv_heads >= 4 else 2.1)
+        dearer = 0.038 * a.kv_heads - alone
+        if singles * a.score_ld / 128 * dearer > 60 and len(runs) <= 8 and any(rows >= 96 and rows > sequences for _, rows, sequences in runs):
+            return runs
+        # mostly single rows, or more keys behind them than behind the portions: as if all rows were single
+        mostly = dearer > 0.005 and (2 * singles >= c.n or singles * a.score_ld >= (c.n - singles) ** 2)
+        return [(0, c.n, c.n if mostly else c.batch)]
+
     def _window_attend(self, a, m, c, qn, y, name):
-        """The two attention passes over the cache for a prepared step (a: WindowArgs with sizes, switches, cache offsets and, if any,
-        gate filled in; qn float [n, heads * maps * dim]; y T, heads * vdim columns).  Pass 1 leaves every row's scores in a scratch [rows,
-        heads, keys a row can see] for pass 2; the step's rows go through the two passes in chunks that keep the scratch within
-        `window_scratch_bytes`."""
-        n, HV, es, heads = c.n, m.heads * m.vdim, y.element_size(), m.heads * getattr(m, "maps", 1)
-        HD, ld_y = heads * m.dim, y.stride(0)
+        """The attention over the cache for a prepared step (a: WindowArgs with sizes, switches, cache offsets and, if any, gate filled in; qn
+        float [n, heads * maps * dim]; y T, heads * vdim columns).  Its two-pass form leaves every row's scores in a scratch [rows, heads, keys a
+        row can see] between the passes; the step's rows go through in chunks that keep the scratch within `window_scratch_bytes`."""
+        HV, es, heads = m.heads * m.vdim, y.element_size(), m.heads * getattr(m, "maps", 1)
+        HD, ld_y, span = heads * m.dim, y.stride(0), getattr(m, "span", m.window)
         f32 = dict(dtype=torch.float32, device=self.device)
-        a.score_ld = self.window_score_ld(getattr(m, "span", m.window), c.max_pos)
+        a.score_ld = self.window_score_ld(span, c.max_pos)
         chunk = max(4, self.window_scratch_bytes // (4 * heads * a.score_ld) // 4 * 4)
-        rows = min(n, chunk)
-        scores = torch.empty(rows, heads, a.score_ld, **f32)
-        ml = torch.empty(rows, heads, a.splits, 2, **f32)
-        o_part = torch.empty(rows, a.splits, HV, **f32)
-        a.scores, a.ml, a.o_part = scores.data_ptr(), ml.data_ptr(), o_part.data_ptr()
         gate, ld_gate = a.gate, a.ld_gate
         with self.timed(name):
-            for at in range(0, n, chunk):
-                a.n = min(chunk, n - at)
-                a.qn, a.y = qn.data_ptr() + 4 * at * HD, y.data_ptr() + es * at * ld_y
-                a.tok_seq, a.tok_pos = c.tok_seq.data_ptr() + 4 * at, c.tok_pos.data_ptr() + 4 * at
-                if gate:
-                    a.gate = gate + es * at * ld_gate
-                H.check(self.lib.b200h_window_attention(C.byref(a)), "window_attention")
+            for first, count, sequences in self._attention_runs(a, c):
+                a.splits = self.window_splits(count, span, c.max_pos)
+                rows = min(count, chunk)
+                scores = torch.empty(rows, heads, a.score_ld, **f32)
+                ml = torch.empty(rows, heads, a.splits, 2, **f32)
+                o_part = torch.empty(rows, a.splits, HV, **f32)
+                a.scores, a.ml, a.o_part = scores.data_ptr(), ml.data_ptr(), o_part.data_ptr()
+                for at in range(first, first + count, chunk):
+                    a.n = min(chunk, first + count - at)
+                    a.sequences = max(1, sequences * a.n // count)
+                    a.qn, a.y = qn.data_ptr() + 4 * at * HD, y.data_ptr() + es * at * ld_y
+                    a.tok_seq, a.tok_pos = c.tok_seq.data_ptr() + 4 * at, c.tok_pos.data_ptr() + 4 * at
+                    if gate:
+                        a.gate = gate + es * at * ld_gate
+                    H.check(self.lib.b200h_window_attention(C.byref(a)), "window_attention")
 
     def conv_attention_mixer(self, i, h, c, run=None):
         """Convolved rotary attention of layer i: one stacked projection (q | k); one kernel convolves every channel over the
@@ -1312,7 +1337,6 @@ class HybridModel:
             H.check(lib.b200h_conv_rope_prep(C.byref(pa)), "conv_rope_prep")
         a = H.WindowArgs()
         a.n, a.heads, a.kv_heads, a.dim, a.vdim, a.block_len, a.window = n, m.heads, m.kv_heads, m.dim, m.vdim, self.block_len, m.window
-        a.splits = self.window_splits(n, m.window, c.max_pos)
         a.scale, a.softcap, a.eps = m.scale, 0.0, self.spec.norm_eps
         a.ld_y = HV
         if m.sink is not None:

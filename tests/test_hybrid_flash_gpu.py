@@ -11,8 +11,9 @@ pytestmark = pytest.mark.gpu
 PAGE = 64
 
 
-def _case(torch, *, rows, heads, kv_heads, dim, vdim, maps=1, window=0, keep=0, chunk=0, sink=False, gate=None, norm=False, seed=0, out_cols=0):
-    """rows: (position of the first row, rows) per sequence -> (result, float64 reference)."""
+def _case(torch, *, rows, heads, kv_heads, dim, vdim, maps=1, window=0, keep=0, chunk=0, sink=False, gate=None, norm=False, seed=0, out_cols=0, sequences=None,
+          one_pass=True):
+    """rows: (position of the first row, rows) per sequence -> (result, float64 reference); checks which form of the attention ran."""
     from lmdeploy_b200 import _hybrid_lib as H
     lib = H.load()
     g = torch.Generator(device="cuda").manual_seed(seed)
@@ -35,7 +36,8 @@ def _case(torch, *, rows, heads, kv_heads, dim, vdim, maps=1, window=0, keep=0, 
     o_part, y = torch.empty(n, 1, hv, device="cuda"), torch.zeros(n, max(out_cols, hv), dtype=torch.bfloat16, device="cuda")
     a = H.WindowArgs(n=n, heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, block_len=PAGE, window=window, splits=1, scale=scale, eps=1e-6, ld=1, chunk=chunk,
                      maps=maps, keep_first=keep, lambda_=lam, out_norm=int(norm), out_scale=0.6, ld_y=y.stride(0), score_ld=ld, dtype=H.BF16,
-                     gate_heads=int(gate == "head"))
+                     gate_heads=int(gate == "head"), sequences=len(rows) if sequences is None else sequences)
+    ml.fill_(float("nan"))                             # the two-pass form leaves every row's maximum and denominator here
     a.q = a.k = a.v = a.qn = qn.data_ptr()
     a.tok_seq, a.tok_pos, a.block_ptrs, a.cu_blocks = seq.data_ptr(), pos.data_ptr(), ptrs.data_ptr(), cu.data_ptr()
     a.v_off = PAGE * KC * 2
@@ -47,6 +49,7 @@ def _case(torch, *, rows, heads, kv_heads, dim, vdim, maps=1, window=0, keep=0, 
     a.stream = torch.cuda.current_stream().cuda_stream
     H.check(lib.b200h_window_attention(C.byref(a)), "window_attention")
     torch.cuda.synchronize()
+    assert bool(ml.isnan().all()) == one_pass
     out, at, cul = [], 0, cu.tolist()
     for s, (p0, r) in enumerate(rows):
         page = pool[order[cul[s]:cul[s + 1]]].double()
@@ -106,3 +109,69 @@ def test_one_long_run_and_many_single_rows():
     import torch
     y, ref = _case(torch, rows=[(0, 1500)] + [(17 * i, 1) for i in range(60)], heads=4, kv_heads=1, dim=128, vdim=128, seed=3)
     assert ((y.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 2e-5).all()
+
+
+@pytest.mark.parametrize("rows,heads,kv_heads,sequences,one_pass", [
+    ([(700 + i, 1) for i in range(128)], 16, 8, None, False),         # a full decode batch: a token fills two of a tile's 128 rows
+    ([(700 + i, 1) for i in range(128)], 16, 8, 0, False),            # the same without the number of sequences
+    ([(700 + i, 1) for i in range(128)], 32, 2, None, True),          # sixteen heads per key/value head
+    ([(900 + i, 2) for i in range(64)], 16, 16, None, False),
+    ([(900 + i, 4) for i in range(32)], 16, 16, None, True),
+    ([(0, 95)], 32, 4, None, False),
+    ([(0, 200)], 16, 8, None, True),
+    ([(0, 128)], 1, 1, None, False),                                  # little work: the plan costs more than it saves
+    ([(900, 1)] * 64 + [(0, 64)], 16, 8, None, False),                # a short prompt beside many single tokens
+    ([(900, 1)] * 64 + [(0, 400)], 16, 8, None, True),
+])
+def test_form_follows_the_rows_of_a_sequence(rows, heads, kv_heads, sequences, one_pass):
+    import torch
+    y, ref = _case(torch, rows=rows, heads=heads, kv_heads=kv_heads, dim=128, vdim=128, sequences=sequences, one_pass=one_pass, seed=4)
+    assert ((y.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 2e-5).all()
+
+
+def _args(H, m, ld):
+    return H.WindowArgs(heads=m.heads, kv_heads=m.kv_heads, dim=m.dim, vdim=m.vdim, maps=m.maps, dtype=H.BF16, score_ld=ld)
+
+
+def test_mixed_steps_send_single_tokens_and_prompts_apart():
+    """HybridModel._window_attend on a step of the engine: 40 sequences that decode, two prompts, 30 more that decode -- three launches, each in its form,
+    and the rows come out as if each had been alone."""
+    import torch
+    from lmdeploy_b200 import _hybrid_lib as H
+    from lmdeploy_b200.turbomind.hybrid import HybridModel, StepArrays
+    from lmdeploy_b200.turbomind.specs import HybridLayerSpec, HybridSpec, WindowAttentionSpec
+    mixer = WindowAttentionSpec(16, 16, 128, 128, 128 ** -0.5, gate=False, qk_norm=False, distance_bias=False, talking_heads=False, bias=False)
+    model = HybridModel(HybridSpec("case", "case", 256, 256, (HybridLayerSpec(mixer, None),), 1e-6, 1, 1, 1.0, block="sandwich", plain_norms=True))
+    shapes, g = model.tensor_shapes(), torch.Generator(device="cuda").manual_seed(3)
+    model.load_weights(lambda name: torch.randn(*shapes[name], generator=g, device="cuda").mul_(shapes[name][-1] ** -0.5).bfloat16())
+    new, hist = [1] * 40 + [150, 90] + [1] * 30, [100 + 3 * i for i in range(40)] + [0, 70] + [333] * 30
+    pages = [(a + b + PAGE - 1) // PAGE for a, b in zip(new, hist)]
+    pool = torch.randn(sum(pages), model.block_bytes // 2, generator=g, device="cuda").bfloat16()
+    i32 = dict(dtype=torch.int32, device="cuda")
+    prefix = lambda x: torch.tensor([sum(x[:i]) for i in range(len(x) + 1)], **i32)  # noqa: E731
+    ptrs = pool.data_ptr() + torch.arange(sum(pages), device="cuda") * model.block_bytes
+    seq, pos = [b for b, r in enumerate(new) for _ in range(r)], [a + i for a, r in zip(hist, new) for i in range(r)]
+    step = dict(n=sum(new), batch=len(new), tok_seq=torch.tensor(seq, **i32), tok_pos=torch.tensor(pos, **i32), cu_q=prefix(new), seq_slot=torch.arange(len(new), **i32),
+                block_ptrs=ptrs, cu_blocks=prefix(pages), state=model.make_state(len(new)), max_pos=max(pos))
+    h = torch.randn(sum(new), 256, generator=g, device="cuda").bfloat16()
+    calls = []
+
+    class Recorder:
+        def __getattr__(self, name):
+            f = getattr(H.load(), name)
+            if name != "b200h_window_attention":
+                return f
+            return lambda ref: calls.append((ref._obj.n, ref._obj.sequences)) or f(ref)
+
+    model.lib = Recorder()
+    together = model.window_mixer(0, h, StepArrays(**step)).clone()
+    assert calls == [(sum(new), len(new))]
+    apart = model.window_mixer(0, h, StepArrays(**step, seq_rows=new))
+    assert calls[1:] == [(40, 40), (240, 2), (30, 30)]
+    calls.clear()
+    few = dict(step, n=242, batch=4, seq_rows=[1, 1, 150, 90])          # two single rows are not worth launches of their own
+    assert model._attention_runs(_args(H, mixer, 512), StepArrays(**few)) == [(0, 242, 4)]
+    most = dict(step, n=110, batch=71, seq_rows=[1] * 70 + [40])        # no portion that the one-pass kernel would take: told as single rows
+    assert model._attention_runs(_args(H, mixer, 512), StepArrays(**most)) == [(0, 110, 110)]
+    # the same float sums in another order under one rounding to bf16 each
+    assert ((together.float() - apart.float()).abs() <= 2.0 ** -7 * together.float().abs() + 2e-5).all()
