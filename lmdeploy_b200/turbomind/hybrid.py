@@ -1289,7 +1289,9 @@ class HybridModel:
     def _window_attend(self, a, m, c, qn, y, name):
         """The attention over the cache for a prepared step (a: WindowArgs with sizes, switches, cache offsets and, if any, gate filled in; qn
         float [n, heads * maps * dim]; y T, heads * vdim columns).  Its two-pass form leaves every row's scores in a scratch [rows, heads, keys a
-        row can see] between the passes; the step's rows go through in chunks that keep the scratch within `window_scratch_bytes`."""
+        row can see] between the passes; the step's rows go through in equal chunks that keep the scratch within `window_scratch_bytes` (equal: a
+        short last one would fall under the one-pass form's least number of rows; 700 rows behind 8000 keys, 24 / 8 heads: 8.0 ms with one of 60
+        rows, 1.2 ms so)."""
         HV, es, heads = m.heads * m.vdim, y.element_size(), m.heads * getattr(m, "maps", 1)
         HD, ld_y, span = heads * m.dim, y.stride(0), getattr(m, "span", m.window)
         f32 = dict(dtype=torch.float32, device=self.device)
@@ -1299,13 +1301,14 @@ class HybridModel:
         with self.timed(name):
             for first, count, sequences in self._attention_runs(a, c):
                 a.splits = self.window_splits(count, span, c.max_pos)
-                rows = min(count, chunk)
+                rows = -(-count // max(1, -(-count // chunk)))
+                rows = min(count, (rows + 3) // 4 * 4)
                 scores = torch.empty(rows, heads, a.score_ld, **f32)
                 ml = torch.empty(rows, heads, a.splits, 2, **f32)
                 o_part = torch.empty(rows, a.splits, HV, **f32)
                 a.scores, a.ml, a.o_part = scores.data_ptr(), ml.data_ptr(), o_part.data_ptr()
-                for at in range(first, first + count, chunk):
-                    a.n = min(chunk, first + count - at)
+                for at in range(first, first + count, max(1, rows)):
+                    a.n = min(rows, first + count - at)
                     a.sequences = max(1, sequences * a.n // count)
                     a.qn, a.y = qn.data_ptr() + 4 * at * HD, y.data_ptr() + es * at * ld_y
                     a.tok_seq, a.tok_pos = c.tok_seq.data_ptr() + 4 * at, c.tok_pos.data_ptr() + 4 * at

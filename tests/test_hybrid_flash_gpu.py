@@ -169,6 +169,10 @@ def test_mixed_steps_send_single_tokens_and_prompts_apart():
     apart = model.window_mixer(0, h, StepArrays(**step, seq_rows=new))
     assert calls[1:] == [(40, 40), (240, 2), (30, 30)]
     calls.clear()
+    model.window_scratch_bytes = 4 * 16 * 512 * 200                     # room for 200 rows of scores: 310 go through as 156 and 154
+    again = model.window_mixer(0, h, StepArrays(**step))
+    assert [n for n, _ in calls] == [156, 154]
+    assert ((together.float() - again.float()).abs() <= 2.0 ** -7 * together.float().abs() + 2e-5).all()
     few = dict(step, n=242, batch=4, seq_rows=[1, 1, 150, 90])          # two single rows are not worth launches of their own
     assert model._attention_runs(_args(H, mixer, 512), StepArrays(**few)) == [(0, 242, 4)]
     most = dict(step, n=110, batch=71, seq_rows=[1] * 70 + [40])        # no portion that the one-pass kernel would take: told as single rows
