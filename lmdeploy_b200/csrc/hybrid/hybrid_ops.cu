@@ -17,6 +17,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <atomic>
 #include <initializer_list>
 #include "../umma.cuh"
 
@@ -762,7 +763,6 @@ __global__ void __launch_bounds__(256, 3) expert_rows_kernel(const T* __restrict
 // of down in 16 us; the float-unit kernels above took 160 us together.  Six blocks per SM with one step of 32 columns each in flight beat
 // fewer blocks with two or four steps (27-30 us), which wait for a whole batch at a time.
 constexpr int kExpertMmaRows = 16, kExpertMmaWarps = 4, kExpertMmaBlocks = 6;
-constexpr int kExpertSteps = 1;
 
 __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1)
 {
@@ -778,8 +778,8 @@ __device__ __forceinline__ uint4 load_once(const bf16* p)              // a weig
     return v;
 }
 
-// NT: groups of eight entries per walk over the weights; U: steps of 32 columns in flight
-template <int MODE, int NT, int U>
+// NT: groups of eight entries per walk over the weights
+template <int MODE, int NT>
 __device__ __forceinline__ void expert_walk(const bf16* __restrict__ x, int x_div, const bf16* __restrict__ wa, const bf16* __restrict__ wb, const int* list,
                                             int live, const float* __restrict__ wts, int K, int R, int r0, void* __restrict__ out_, float* red)
 {
@@ -797,36 +797,24 @@ __device__ __forceinline__ void expert_walk(const bf16* __restrict__ x, int x_di
 #pragma unroll
         for (int q = 0; q < NT; ++q) acc[m][q][0] = acc[m][q][1] = acc[m][q][2] = acc[m][q][3] = 0.f;
 #pragma unroll 1
-    for (int k = 0; k < slice; k += 32 * U) {
-        uint4 a[U][DUAL ? 4 : 2], b[U][NT];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int at = k + 32 * u;
-            if (at < slice) {
-                a[u][0] = load_once(wa + ra + at);
-                a[u][1] = load_once(wa + rb + at);
-                if (DUAL) {
-                    a[u][DUAL ? 2 : 0] = load_once(wb + ra + at);
-                    a[u][DUAL ? 3 : 0] = load_once(wb + rb + at);
-                }
-            }
+    for (int k = 0; k < slice; k += 32) {
+        uint4 a[DUAL ? 4 : 2], b[NT];
+        a[0] = load_once(wa + ra + k);
+        a[1] = load_once(wa + rb + k);
+        if (DUAL) {
+            a[DUAL ? 2 : 0] = load_once(wb + ra + k);
+            a[DUAL ? 3 : 0] = load_once(wb + rb + k);
         }
 #pragma unroll
-        for (int u = 0; u < U; ++u)
-            if (k + 32 * u < slice)
+        for (int q = 0; q < NT; ++q) b[q] = *reinterpret_cast<const uint4*>(px[q] + k);
 #pragma unroll
-                for (int q = 0; q < NT; ++q) b[u][q] = *reinterpret_cast<const uint4*>(px[q] + k + 32 * u);
+        for (int m = 0; m < (DUAL ? 2 : 1); ++m)
 #pragma unroll
-        for (int u = 0; u < U; ++u)
-            if (k + 32 * u < slice)
-#pragma unroll
-                for (int m = 0; m < (DUAL ? 2 : 1); ++m)
-#pragma unroll
-                    for (int q = 0; q < NT; ++q) {
-                        const uint4 lo = a[u][2 * m], hi = a[u][2 * m + 1];
-                        mma_bf16(acc[m][q], lo.x, hi.x, lo.y, hi.y, b[u][q].x, b[u][q].y);
-                        mma_bf16(acc[m][q], lo.z, hi.z, lo.w, hi.w, b[u][q].z, b[u][q].w);
-                    }
+            for (int q = 0; q < NT; ++q) {
+                const uint4 lo = a[2 * m], hi = a[2 * m + 1];
+                mma_bf16(acc[m][q], lo.x, hi.x, lo.y, hi.y, b[q].x, b[q].y);
+                mma_bf16(acc[m][q], lo.z, hi.z, lo.w, hi.w, b[q].z, b[q].w);
+            }
     }
     // the warps' quarters, summed in order
     __syncthreads();
@@ -853,7 +841,7 @@ __device__ __forceinline__ void expert_walk(const bf16* __restrict__ x, int x_di
     }
 }
 
-template <int MODE, int NT, int U>
+template <int MODE, int NT>
 __global__ void __launch_bounds__(32 * kExpertMmaWarps, kExpertMmaBlocks) expert_mma_kernel(const bf16* __restrict__ x, int x_div, const bf16* __restrict__ wa, const bf16* __restrict__ wb,
                                                                           const int* __restrict__ ids, int entries, const float* __restrict__ wts, int K, int R,
                                                                           void* __restrict__ out_)
@@ -882,24 +870,27 @@ __global__ void __launch_bounds__(32 * kExpertMmaWarps, kExpertMmaBlocks) expert
         }
         const int live = min(8 * NT, seen - done);
         if (live <= 0) break;
-        expert_walk<MODE, NT, U>(x, x_div, wa, wb, list, live, wts, K, R, r0, out_, red);
+        expert_walk<MODE, NT>(x, x_div, wa, wb, list, live, wts, K, R, r0, out_, red);
         done += live;
         if (done >= seen) break;
     }
 }
 
-// NT by the entries an expert has on average: what does not fit one walk over the weights reads them again (from the L2)
+// NT by the entries an expert has on average: what does not fit one walk over the weights reads them again (from the L2), and a wider walk
+// costs registers.  Measured, us with 1 / 2 / 4 groups: 8 experts of 2048 x 2048, two chosen: 4 entries each 50 / 50 / 78, 5: 64 / 50 / 77, 12: 87 /
+// 67 / 79, 14: 92 / 68 / 79, 24: 135 / 96 / 83; of 4096 x 1408: 12: 110 / 70 / 84, 14: 134 / 91 / 85; 64 experts of 2048 x 1408, six chosen: 3.75:
+// 212 / 217 / 263, 4.5: 217 / 220 / 268, 12: 369 / 258 / 288, 18: 496 / 341 / 309.
 template <int MODE>
 static void launch_expert_mma(const void* x, int x_div, const void* wa, const void* wb, const void* ids, int entries, const float* wts, int experts, int K, int R,
                               void* out, cudaStream_t st)
 {
     const dim3 grid((R + kExpertMmaRows - 1) / kExpertMmaRows, experts);
-#define B200H_EXPERT_MMA(NT, U)                                                                                                           \
-    expert_mma_kernel<MODE, NT, U><<<grid, 32 * kExpertMmaWarps, 0, st>>>((const bf16*)x, x_div, (const bf16*)wa, (const bf16*)wb, (const int*)ids, entries, wts, \
+#define B200H_EXPERT_MMA(NT)                                                                                                              \
+    expert_mma_kernel<MODE, NT><<<grid, 32 * kExpertMmaWarps, 0, st>>>((const bf16*)x, x_div, (const bf16*)wa, (const bf16*)wb, (const int*)ids, entries, wts, \
                                                                           K, R, out)
-    if (entries <= 4 * experts) B200H_EXPERT_MMA(1, kExpertSteps);
-    else if (entries <= 12 * experts) B200H_EXPERT_MMA(2, kExpertSteps);
-    else B200H_EXPERT_MMA(4, kExpertSteps);
+    if (entries <= 4 * experts) B200H_EXPERT_MMA(1);
+    else if (entries <= 12 * experts) B200H_EXPERT_MMA(2);
+    else B200H_EXPERT_MMA(4);
 #undef B200H_EXPERT_MMA
 }
 
@@ -1499,15 +1490,23 @@ static bool flash_attention_pays(const b200h_window_args* a)
     return a->n >= kFaMinRows && one < two;
 }
 
+constexpr int kMaxDevices = 64;
+
 template <int D, int MAPS, int V>
 static int launch_flash(const FlashArgs& a, cudaStream_t st)
 {
+    const auto kernel = flash_attention_kernel<D, MAPS, V>;
+    static std::atomic<int> sms_of[kMaxDevices];                        // SMs of a device on which the kernel may use its shared memory; 0: not asked yet
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const auto kernel = flash_attention_kernel<D, MAPS, V>;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FlashShape<D, MAPS, V>::kSmem) != cudaSuccess)
-        return fail(B200H_ERR_UNSUPPORTED, "window_attention: shared memory of the tensor-core form");
+    const bool slot = dev >= 0 && dev < kMaxDevices;
+    if (slot) sms = sms_of[dev].load(std::memory_order_acquire);
+    if (sms == 0) {
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FlashShape<D, MAPS, V>::kSmem) != cudaSuccess)
+            return fail(B200H_ERR_UNSUPPORTED, "window_attention: shared memory of the tensor-core form");
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (slot) sms_of[dev].store(sms, std::memory_order_release);
+    }
     const int tokens = 128 / (a.heads / a.kv_heads);
     flash_plan_kernel<<<1, 1024, 0, st>>>(a, MAPS == 2 ? tokens : 2 * tokens);
     kernel<<<sms, kFaThreads, FlashShape<D, MAPS, V>::kSmem, st>>>(a);
