@@ -171,7 +171,8 @@ B200_API int b200_process_kv(const b200_attention_params* params);
  * q_len and history_len + q_len per sequence; `out` is token-major [token_num, num_heads * 128] (out_packed_mt must be
  * 0); workspace = b200_prefill_attention_workspace_bytes(token_num, num_heads), most of it room for the partial results of
  * keys that several SMs share (token_num * num_heads * 256 bytes, the rotated queries alone, are enough for the same results
- * with a piece per SM); `plan`, `max_k_len` are not used. */
+ * with a piece per SM); `plan` is not used; `max_k_len`, if positive, is taken for the longest context of the step and chooses among
+ * forms of the same result (any of them is right for any length). */
 B200_API size_t b200_prefill_attention_workspace_bytes(int token_num, int num_heads);
 B200_API int b200_prefill_attention(const b200_attention_params* params);
 

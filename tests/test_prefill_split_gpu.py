@@ -10,20 +10,26 @@ from test_prefill_attention_gpu import _prefill_case
 pytestmark = pytest.mark.gpu
 
 
-class _Workspace:
-    """The library with a smaller workspace: `more` bytes beyond the rotated queries, the least that the operator takes."""
+class _Call:
+    """The library with another workspace (`more` bytes beyond the rotated queries, the least that the operator takes; None: all it asks for) and another
+    word about the longest context."""
 
-    def __init__(self, lib, more):
-        self.lib, self.more = lib, more
+    def __init__(self, lib, more, keys):
+        self.lib, self.more, self.keys = lib, more, keys
 
     def __getattr__(self, name):
         return getattr(self.lib, name)
 
     def b200_prefill_attention_workspace_bytes(self, tokens, heads):
-        return tokens * heads * 256 + self.more
+        return self.lib.b200_prefill_attention_workspace_bytes(tokens, heads) if self.more is None else tokens * heads * 256 + self.more
+
+    def b200_prefill_attention(self, ref):
+        ref._obj.max_k_len = self.keys
+        return self.lib.b200_prefill_attention(ref)
 
 
-@pytest.mark.parametrize("more", [None, 0, 20000])
+# shared keys; whole pieces for want of room; whole pieces and the short form for what the caller says of the contexts (not true here: any form is right)
+@pytest.mark.parametrize("more,keys", [(None, 0), (0, 0), (20000, 0), (None, 200), (None, 128)])
 @pytest.mark.parametrize("kv_bits,dtype,heads,q_lens,hists", [
     (8, F16, (8, 2), [127, 128, 129, 64, 65, 1], [0, 0, 0, 64, 63, 127]),
     (16, F16, (4, 1), [3, 40], [1500, 700]),
@@ -31,8 +37,8 @@ class _Workspace:
     (16, BF16, (7, 1), [19, 37, 300], [0, 128, 127]),
     (8, BF16, (2, 2), [257, 1], [255, 900]),
 ])
-def test_cut_work_matches_oracle(lib, kv_bits, dtype, heads, q_lens, hists, more):
-    got, ref, pool, ref_pool = _prefill_case(lib if more is None else _Workspace(lib, more), q_lens=q_lens, hists=hists, Hq=heads[0], Hkv=heads[1], kv_bits=kv_bits,
+def test_cut_work_matches_oracle(lib, kv_bits, dtype, heads, q_lens, hists, more, keys):
+    got, ref, pool, ref_pool = _prefill_case(_Call(lib, more, keys), q_lens=q_lens, hists=hists, Hq=heads[0], Hkv=heads[1], kv_bits=kv_bits,
                                              dtype=dtype, seed=sum(q_lens))
     assert np.array_equal(pool, ref_pool)
     # P is rounded to T before P.V and the output is rounded to T (half an ulp each, 2^-12 / 2^-9 relative to values up to 4): as for the whole prompts
