@@ -815,26 +815,6 @@ extern "C" int b200_linear_forward(const b200_linear_desc* d, const void* x, int
     return forward_packed(d, w.xp, mt, m, y, ldy, epilogue, 0, 0, w.partials, w.counters, st);
 }
 
-namespace b200 {
-
-bool linear_reads_rows(const b200_linear_desc* d, int m)
-{
-    return !validate_desc(d) && thin_pays(d, m);
-}
-
-int linear_forward_rows(const b200_linear_desc* d, const void* x, int64_t ldx, int m, void* y, int64_t ldy, int epilogue, int out_packed_mt, void* stream)
-{
-    if (int e = validate_desc(d)) {
-        return e;
-    }
-    if (!thin_fits(d, m) || !d->prepared || !x || !y) {
-        return fail(B200_ERR_INVALID_ARG, "linear_forward_rows: bad arguments");
-    }
-    return forward_thin(d, thin_shape(d, m), x, ldx, m, y, ldy, epilogue, out_packed_mt > 0 ? 1 : 0, out_packed_mt, (cudaStream_t)stream);
-}
-
-}  // namespace b200
-
 extern "C" int b200_linear_forward_packed(const b200_linear_desc* d, const void* xp, int mt, int m, void* y,
                                           int64_t ldy, int epilogue, int out_packed_mt, void* workspace,
                                           size_t workspace_bytes, void* stream)

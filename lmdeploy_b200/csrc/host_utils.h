@@ -1,6 +1,5 @@
 // Host-side helpers shared by the C-ABI translation units: thread-local error text, launch checks.
 #pragma once
-#include "../../include/b200_turbomind.h"
 #include <cuda_runtime.h>
 #include <cstdio>
 #include <cstdlib>
@@ -73,11 +72,6 @@ inline int current_device()
     cudaGetDevice(&dev);
     return dev >= 0 && dev < kMaxDevices ? dev : 0;
 }
-
-// gemm.cu: does a layer of m tokens read row-major activations (linear_forward_rows) or the packed tile layout?  Whatever produces
-// the activations asks before it writes them; the answer depends on the layer, m and the loaded launch plans alone.
-bool linear_reads_rows(const ::b200_linear_desc* d, int m);
-int  linear_forward_rows(const ::b200_linear_desc* d, const void* x, int64_t ldx, int m, void* y, int64_t ldy, int epilogue, int out_packed_mt, void* stream);
 
 #define B200_CUDA_TRY(expr)                                                                                            \
     do {                                                                                                               \

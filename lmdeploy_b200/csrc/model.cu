@@ -6,7 +6,7 @@
 //   Generation::Forward (greedy)      src/turbomind/generation/generation.cc:247-293 )
 // One call enqueues the whole step on a stream with no host synchronisation, so the caller can capture it in a
 // CUDA graph.  Activations between kernels live in the UMMA K-major tile layout so that every GEMM's B operand
-// is one contiguous TMA bulk copy, or row-major in front of the layers that take few tokens in place (linear_thin.cuh).
+// is one contiguous TMA bulk copy.
 #include <cstdlib>
 #include "../../include/b200_turbomind.h"
 #include "host_utils.h"
@@ -298,20 +298,11 @@ static int run_step(b200_model* m, const b200_step_inputs* in, int R, bool chunk
     const int qkv_dim = (c.num_heads + 2 * c.num_kv_heads) * c.head_dim;
     const int es      = 2;
     const int L       = c.num_layers;
-    // layout of a layer's input: row-major (0) where the layer reads it so, else the packed tiles of MT tokens.  Asked once per use:
-    // launch plans may be loaded meanwhile, and whoever writes and whoever reads have to agree.
-    auto layout = [&](const b200_linear_desc& d) { return linear_reads_rows(&d, R) ? 0 : MT; };
-    auto linear = [&](const b200_linear_desc& d, int in_mt, const void* x, void* y, int ldy, int epilogue, int out_mt) {
-        return in_mt == 0 ? linear_forward_rows(&d, x, d.input_dim, R, y, ldy, epilogue, out_mt, stream) :
-                            b200_linear_forward_packed(&d, x, MT, R, y, ldy, epilogue, out_mt, m->lin_ws, m->lin_ws_bytes, stream);
-    };
-    const bool fuse    = !m->comm && m->fuse_norm;      // the fused epilogue belongs to the packed kernel
     void*     o_buf   = m->o_x[0] ? m->o_x[0] : m->o;   // wo output (exchange half 0 under TP)
     void*     o_buf2  = m->o_x[1] ? m->o_x[1] : m->o;   // w2 output (exchange half 1 under TP)
 
     TRY_T(0, b200_embedding_lookup(m->residual, m->embedding, in->token_ids, R, c.hidden, c.embedding_rows, c.dtype, stream));
-    int xp_mt = layout(m->layers[0].qkv);                // layout of m->xp at this point
-    TRY_T(0, b200_rmsnorm(m->xp, xp_mt, m->residual, m->layers[0].attn_norm, R, c.hidden, c.norm_eps, c.dtype, stream));
+    TRY_T(0, b200_rmsnorm(m->xp, MT, m->residual, m->layers[0].attn_norm, R, c.hidden, c.norm_eps, c.dtype, stream));
     if (!chunk) {
         TRY_T(0, b200_decode_attention_plan(m->plan, in->cu_k_len, in->finished, B, stream));
     }
@@ -323,8 +314,7 @@ static int run_step(b200_model* m, const b200_step_inputs* in, int R, bool chunk
             return fail(B200_ERR_STATE, "decode_step: layer weights not set");
         }
         // ---- attention block ----
-        TRY_T(1, linear(W.qkv, xp_mt, m->xp, m->qkv, qkv_dim, 0, 0));
-        const int o_mt = fuse ? MT : layout(W.wo), ffn_mt = layout(W.w13), act_mt = fuse ? MT : layout(W.w2);
+        TRY_T(1, b200_linear_forward_packed(&W.qkv, m->xp, MT, R, m->qkv, qkv_dim, 0, 0, m->lin_ws, m->lin_ws_bytes, stream));
         if (W.q_norm && W.k_norm) {
             TRY_T(1, b200_qk_rmsnorm(m->qkv, qkv_dim, W.q_norm, W.k_norm, R, c.num_heads, c.num_kv_heads, c.head_dim, c.norm_eps,
                                      c.dtype, stream));
@@ -348,23 +338,23 @@ static int run_step(b200_model* m, const b200_step_inputs* in, int R, bool chunk
         a.inv_sqrt_dh = c.inv_sqrt_dh, a.window_size = 0;
         a.rope = c.rope, a.quant_policy = c.quant_policy, a.dtype = c.dtype;
         a.workspace = m->attn_ws, a.workspace_bytes = m->attn_ws_bytes;
-        a.plan = m->plan, a.rope_table = m->rope_table, a.out_packed_mt = o_mt, a.stream = stream;
+        a.plan = m->plan, a.rope_table = m->rope_table, a.out_packed_mt = MT, a.stream = stream;
         if (!chunk) {
             TRY_T(2, b200_decode_attention(&a));
         }
         else {
-            // row-major; where the wo GEMM reads the packed layout, by way of the (currently idle) GEMM output buffer
+            // row-major into the (currently idle) GEMM output buffer, then into the packed layout the wo GEMM reads
             const int attn_dim = c.num_heads * c.head_dim;
-            a.out = o_mt ? m->o : m->attn_xp, a.out_packed_mt = 0, a.plan = nullptr;
+            a.out = m->o, a.out_packed_mt = 0, a.plan = nullptr;
             TRY_T(2, b200_prefill_attention(&a));
-            if (o_mt) TRY_T(2, b200_pack_activations(m->o, attn_dim, R, attn_dim, MT, c.dtype, m->attn_xp, stream));
+            TRY_T(2, b200_pack_activations(m->o, attn_dim, R, attn_dim, MT, c.dtype, m->attn_xp, stream));
         }
         // wo GEMM + AllreduceResidualRMSnorm #1 (unified_decoder.cc:278-287).  Single GPU: the residual add and the
         // RMSNorm are fused into the GEMM's split-K epilogue when the launch plan has one.
         bool fused1 = false;
-        if (fuse) {
+        if (!m->comm && m->fuse_norm) {
             const int rc = b200_linear_forward_packed_residual_rmsnorm(&W.wo, m->attn_xp, MT, R, m->residual, W.ffn_norm,
-                                                                       c.norm_eps, m->xp, ffn_mt, m->lin_ws, m->lin_ws_bytes,
+                                                                       c.norm_eps, m->xp, MT, m->lin_ws, m->lin_ws_bytes,
                                                                        stream);
             if (rc == 0) {
                 fused1 = true;
@@ -374,24 +364,24 @@ static int run_step(b200_model* m, const b200_step_inputs* in, int R, bool chunk
             }
         }
         if (!fused1) {
-            TRY_T(3, linear(W.wo, o_mt, m->attn_xp, o_buf, c.hidden, 0, 0));
+            TRY_T(3, b200_linear_forward_packed(&W.wo, m->attn_xp, MT, R, o_buf, c.hidden, 0, 0, m->lin_ws, m->lin_ws_bytes, stream));
             if (m->comm) {
-                TRY_T(4, b200_comm_allreduce_residual_rmsnorm(m->comm, m->xp, ffn_mt, m->residual, o_buf, W.ffn_norm, nullptr, R,
+                TRY_T(4, b200_comm_allreduce_residual_rmsnorm(m->comm, m->xp, MT, m->residual, o_buf, W.ffn_norm, nullptr, R,
                                                               c.hidden, c.norm_eps, c.dtype, stream));
             }
             else {
-                TRY_T(4, b200_residual_rmsnorm(m->xp, ffn_mt, m->residual, o_buf, W.ffn_norm, nullptr, R, c.hidden, c.norm_eps,
+                TRY_T(4, b200_residual_rmsnorm(m->xp, MT, m->residual, o_buf, W.ffn_norm, nullptr, R, c.hidden, c.norm_eps,
                                                c.dtype, stream));
             }
         }
         // ---- FFN block ----
-        TRY_T(5, linear(W.w13, ffn_mt, m->xp, m->act_xp, c.inter_size, 1, act_mt));
-        xp_mt = layout(l + 1 < L ? m->layers[l + 1].qkv : m->lm_head);
+        TRY_T(5, b200_linear_forward_packed(&W.w13, m->xp, MT, R, m->act_xp, c.inter_size, 1, MT, m->lin_ws, m->lin_ws_bytes,
+                                       stream));
         const void* next_norm = (l + 1 < L) ? m->layers[l + 1].attn_norm : m->final_norm;
         bool        fused2    = false;
-        if (fuse) {
+        if (!m->comm && m->fuse_norm) {
             const int rc = b200_linear_forward_packed_residual_rmsnorm(&W.w2, m->act_xp, MT, R, m->residual, next_norm,
-                                                                       c.norm_eps, m->xp, xp_mt, m->lin_ws, m->lin_ws_bytes,
+                                                                       c.norm_eps, m->xp, MT, m->lin_ws, m->lin_ws_bytes,
                                                                        stream);
             if (rc == 0) {
                 fused2 = true;
@@ -401,19 +391,20 @@ static int run_step(b200_model* m, const b200_step_inputs* in, int R, bool chunk
             }
         }
         if (!fused2) {
-            TRY_T(6, linear(W.w2, act_mt, m->act_xp, o_buf2, c.hidden, 0, 0));
+            TRY_T(6, b200_linear_forward_packed(&W.w2, m->act_xp, MT, R, o_buf2, c.hidden, 0, 0, m->lin_ws, m->lin_ws_bytes, stream));
             if (m->comm) {
-                TRY_T(7, b200_comm_allreduce_residual_rmsnorm(m->comm, m->xp, xp_mt, m->residual, o_buf2, next_norm, nullptr, R,
+                TRY_T(7, b200_comm_allreduce_residual_rmsnorm(m->comm, m->xp, MT, m->residual, o_buf2, next_norm, nullptr, R,
                                                               c.hidden, c.norm_eps, c.dtype, stream));
             }
             else {
-                TRY_T(7, b200_residual_rmsnorm(m->xp, xp_mt, m->residual, o_buf2, next_norm, nullptr, R, c.hidden, c.norm_eps, c.dtype,
+                TRY_T(7, b200_residual_rmsnorm(m->xp, MT, m->residual, o_buf2, next_norm, nullptr, R, c.hidden, c.norm_eps, c.dtype,
                                                stream));
             }
         }
     }
     // PostEmbedding (language_model.cc:285-335) + greedy sampling
-    TRY_T(8, linear(m->lm_head, xp_mt, m->xp, m->logits, c.vocab, 0, 0));
+    TRY_T(8, b200_linear_forward_packed(&m->lm_head, m->xp, MT, R, m->logits, c.vocab, 0, 0, m->lin_ws, m->lin_ws_bytes,
+                                   stream));
     if (in->out_tokens) {
         // c.vocab is the per-rank lm_head width padded to a multiple of 128; only the columns below the real vocabulary
         // size (= rows of the embedding table) may be sampled (sampling.cc:132: vocab_size, not vocab_size_padded)
