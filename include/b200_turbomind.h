@@ -200,6 +200,10 @@ B200_API int b200_decode_attention_grid(int quant_policy, int dtype);
  * `prepared` is library-owned layout (b200_linear_prepared_bytes bytes); `bias` may be NULL.
  * Workspace must be zero-filled ONCE before its first use (split-K arrival counters live in it; the
  * kernels leave them zero).
+ * Order on a stream: calls that use a layer may follow its b200_linear_prepare directly.  b200_linear_forward reads nothing before all
+ * earlier work of the stream has completed.  The _packed calls and a model's steps fetch weights while the kernel ahead of them still
+ * runs: where a kernel other than b200_linear_prepare's writes `prepared`, wait for it (an event, a copy, any call that is not a
+ * kernel) before the first of them.
  * ---------------------------------------------------------------------------------------------- */
 typedef struct {
     int         input_dim;     /* K */

@@ -184,14 +184,14 @@ __global__ void prepare_dense_kernel(T* dst, const T* w, int K, int N, int trans
     }
 }
 
-// activations: X [M][ldx] row-major -> XP [K/8][MT][8]; rows >= M are zero
+// activations: X [M][ldx] row-major -> XP [K/8][MT][8]; rows >= M are zero.  It lets the GEMM behind it start, which
+// fetches weights at once, only when everything ahead of it in the stream has completed: whatever kernel wrote the weights, they are there
 template<class T>
 __global__ void pack_x_kernel(T* xp, const T* x, int M, int MT, int K, int64_t ldx)
 {
     const size_t n16 = (size_t)(K / 8) * MT;  // 16-byte units
-    // the GEMM behind it may start fetching its weights now; x may be the previous kernel's output and xp what it reads
-    pdl_launch_dependents();
     pdl_wait();
+    pdl_launch_dependents();
     for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < n16; idx += (size_t)gridDim.x * blockDim.x) {
         const int tok = (int)(idx % MT);
         const int k8  = (int)(idx / MT);
@@ -202,6 +202,10 @@ __global__ void pack_x_kernel(T* xp, const T* x, int M, int MT, int K, int64_t l
         reinterpret_cast<uint4*>(xp)[idx] = v;
     }
 }
+
+// Last launch of a prepare.  The kernels that read prepared weights start before the kernel ahead of them has ended (programmatic
+// dependent launch) and fetch weights at once; behind this one, which writes nothing and begins when the weights are complete, they may
+__global__ void prepared_kernel() {}
 
 constexpr int kMaxSplits = 16;
 
@@ -655,6 +659,7 @@ extern "C" int b200_linear_prepare(const b200_linear_desc* d, const void* weight
         prepare_dense_kernel<uint16_t><<<2048, 256, 0, st>>>((uint16_t*)prepared, (const uint16_t*)weight, K, N,
                                                              weight_is_transposed);
     }
+    prepared_kernel<<<1, 1, 0, st>>>();
     return check_launch("prepare kernel");
 }
 

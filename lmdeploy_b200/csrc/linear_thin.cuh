@@ -119,6 +119,9 @@ __global__ void __launch_bounds__(kThinThreads, 2) linear_thin_kernel(const Para
             }
         }
     };
+    // from here on: weights (the kernel ahead may be the one that writes them: no pack stands between), activations, an output that
+    // an earlier kernel may still read
+    pdl_wait();
 #pragma unroll
     for (int s = 0; s < DEPTH; ++s) {
         if (kw + s * KW < kgs) {
@@ -129,7 +132,6 @@ __global__ void __launch_bounds__(kThinThreads, 2) linear_thin_kernel(const Para
     if constexpr (FMT == kU4 && std::is_same<T, half>::value) {
         dn = __ldg(p.u4_fast) != 0;
     }
-    pdl_wait();  // from here on: activations of the previous kernel, an output that it may still read
     if (warp == 0) {
         for (int j = 0; j < min(tp.stages, steps); ++j) {
             fetch_x(j);
