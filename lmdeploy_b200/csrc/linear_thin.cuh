@@ -12,8 +12,7 @@
 //     uses the same ones, so nothing is shuffled;
 //   * X is read in place (row-major) by bulk copies into a ring of shared memory, kw k-groups of every token per stage, and from
 //     there by the lane that needs it.
-// u4 weights become the same T(fma(q, s, t)) as in the tcgen05 kernel; e4m3 weights enter the product as they are and a group's
-// fp32 sum is multiplied by its scale (the tcgen05 kernel rounds weight * scale to T first): no error is larger than there.
+// u4 weights become the same T(fma(q, s, t)) as in the tcgen05 kernel, e4m3 weights the same T(weight * scale).
 //
 // Measured (us, captured calls, tcgen05 kernel without its pack launch -> this kernel): u4 4096 x 6144, m 1: 11.8 -> 6.4; 4096 x
 // 4096: 11.0 -> 4.7; 14336 x 4096: 15.5 -> 11.2; 1024 x 1536: 7.0 -> 2.1; fp8 8192 x 7168, m 8: 21.8 -> 16.1; dense 14336 x 4096, m 1:
@@ -60,13 +59,26 @@ B200_DEVICE uint32_t e4m3x2_to(uint32_t x)  // two e4m3 bytes (low half of x) ->
     return h2;
 }
 
+// the T product of the tcgen05 kernel's weights: exact, rounded once
+template<class T>
+B200_DEVICE uint32_t mul2(uint32_t a, uint32_t b)
+{
+    uint32_t d;
+    if constexpr (std::is_same<T, nv_bfloat16>::value) {
+        asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    }
+    else {
+        asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    }
+    return d;
+}
+
 template<class T, int FMT, int RT, int NT, int DEPTH>
 __global__ void __launch_bounds__(kThinThreads, 2) linear_thin_kernel(const Params p, const ThinParams tp)
 {
     using Ops            = TypeOps<T>;
     constexpr int  LW    = FMT == kU4 ? 1 : FMT == kDense ? 4 : 2;  // 32-byte loads per (16 rows, k-group) and lane
     constexpr int  WB    = block_bytes_of(FMT);
-    constexpr bool kPost = FMT == kFp8Col;                          // scales applied to a group's sums
     static_assert(WB % 32 == 0, "a lane's 32 bytes of any block are aligned");
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ uint64_t bar_full[kThinMaxStages], bar_empty[kThinMaxStages];
@@ -149,15 +161,6 @@ __global__ void __launch_bounds__(kThinThreads, 2) linear_thin_kernel(const Para
     // the 16-byte chunk of 8 k's that unit `i` (0..3) of this lane's k's in the group stands for
     auto chunk   = [&](int i) { return FMT == kU4 ? t * 4 + i : FMT == kDense ? i * 4 + t : ((i >> 1) * 4 + t) * 2 + (i & 1); };
     auto compute = [&](auto DN, int st, uint32_t xsm) {
-        float part[kPost ? RT : 1][NT][4];
-        if constexpr (kPost) {
-#pragma unroll
-            for (int r = 0; r < RT; ++r)
-#pragma unroll
-                for (int j = 0; j < NT; ++j)
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) part[r][j][c] = 0.f;
-        }
 #pragma unroll
         for (int i = 0; i < 4; ++i) {  // 8 k's of each of the two rows
             uint4 x[NT];
@@ -190,11 +193,12 @@ __global__ void __launch_bounds__(kThinThreads, 2) linear_thin_kernel(const Para
                     for (int e = 0; e < 4; ++e) a0[e] = w[st][r][i][e], a1[e] = w[st][r][i][4 + e];
                 }
                 else {
+                    const uint32_t s0 = __byte_perm(par[st][r].x, 0, 0x1010), s1 = __byte_perm(par[st][r].y, 0, 0x1010);
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
                         const uint32_t q0 = w[st][r][i >> 1][(i & 1) * 2 + (e >> 1)], q1 = w[st][r][i >> 1][4 + (i & 1) * 2 + (e >> 1)];
-                        a0[e] = e4m3x2_to<T>(e & 1 ? q0 >> 16 : q0 & 0xffffu);
-                        a1[e] = e4m3x2_to<T>(e & 1 ? q1 >> 16 : q1 & 0xffffu);
+                        a0[e] = mul2<T>(e4m3x2_to<T>(e & 1 ? q0 >> 16 : q0 & 0xffffu), s0);
+                        a1[e] = mul2<T>(e4m3x2_to<T>(e & 1 ? q1 >> 16 : q1 & 0xffffu), s1);
                     }
                 }
 #pragma unroll
@@ -203,21 +207,8 @@ __global__ void __launch_bounds__(kThinThreads, 2) linear_thin_kernel(const Para
 #pragma unroll
                     for (int j = 0; j < NT; ++j) {
                         const uint32_t b[2] = {h ? x[j].z : x[j].x, h ? x[j].w : x[j].y};
-                        Ops::mma16816(kPost ? part[kPost ? r : 0][j] : acc[r][j], a, b);
+                        Ops::mma16816(acc[r][j], a, b);
                     }
-                }
-            }
-        }
-        if constexpr (kPost) {
-#pragma unroll
-            for (int r = 0; r < RT; ++r) {
-                const float s0 = Ops::to_f32(Ops::from_bits((uint16_t)par[st][r].x)), s1 = Ops::to_f32(Ops::from_bits((uint16_t)par[st][r].y));
-#pragma unroll
-                for (int j = 0; j < NT; ++j) {
-                    acc[r][j][0] = fmaf(s0, part[r][j][0], acc[r][j][0]);
-                    acc[r][j][1] = fmaf(s0, part[r][j][1], acc[r][j][1]);
-                    acc[r][j][2] = fmaf(s1, part[r][j][2], acc[r][j][2]);
-                    acc[r][j][3] = fmaf(s1, part[r][j][3], acc[r][j][3]);
                 }
             }
         }
