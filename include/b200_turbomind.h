@@ -236,7 +236,15 @@ B200_API int b200_linear_forward_packed_residual_rmsnorm(const b200_linear_desc*
                                                 void* residual, const void* norm_weight, float eps, void* out,
                                                 int out_packed_mt, void* workspace, size_t workspace_bytes,
                                                 void* stream);
-/* launch plan of a shape (host only; no device work): out8 = {n-tiles per CTA, K splits, W ring, X ring, TMEM A slots,
+/* Which kernel a layer's call of m tokens runs (host only; no device work), or a negative b200_status:
+ *   B200_LINEAR_TILES       the tcgen05 kernel that b200_linear_plan describes
+ *   B200_LINEAR_FEW_TOKENS  b200_linear_forward only, up to 24 tokens: row-major activations, mma.sync, K not split; formats 0, 1 and 3 with
+ *                           `prepared` on a 32-byte boundary, and x and y that do not overlap (calls where they do run the others)
+ *   B200_LINEAR_HEAD        dense, more than 64 tokens, many output features: a persistent tcgen05 kernel
+ * packed: the call is b200_linear_forward_packed.  A loaded plan of the shape (below) always selects the first. */
+enum { B200_LINEAR_TILES = 0, B200_LINEAR_FEW_TOKENS = 1, B200_LINEAR_HEAD = 2 };
+B200_API int b200_linear_kernel(const b200_linear_desc* desc, int m, int packed);
+/* launch plan of a shape in the first of these kernels (host only; no device work): out8 = {n-tiles per CTA, K splits, W ring, X ring, TMEM A slots,
  * TMEM columns, first A column, dynamic shared memory bytes}.  A pure function of (format, K, N, padded m). */
 B200_API int b200_linear_plan(const b200_linear_desc* desc, int m, int* out8);
 /* Tuned launch plans -- the counterpart of the reference's GEMM tuning cache (gemm::Gemm::Export / Import,

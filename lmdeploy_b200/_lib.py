@@ -129,6 +129,8 @@ def load():
         C.c_void_p, C.c_size_t, C.c_void_p]
     lib.b200_linear_plan.argtypes = [C.POINTER(LinearDesc), C.c_int, C.POINTER(C.c_int)]
     lib.b200_linear_plan.restype = C.c_int
+    lib.b200_linear_kernel.argtypes = [C.POINTER(LinearDesc), C.c_int, C.c_int]
+    lib.b200_linear_kernel.restype = C.c_int
     lib.b200_linear_load_plans.argtypes = [C.c_char_p]
     lib.b200_linear_load_plans.restype = C.c_int
     lib.b200_pack_activations.argtypes = [C.c_void_p, C.c_int64, C.c_int, C.c_int, C.c_int, C.c_int, C.c_void_p,

@@ -416,10 +416,16 @@ static int launch(const Params& p, int smem, cudaStream_t st)
 // 64.  Up to 64 tokens the tile of X is half as large and half of the rows here are padding: a model's step with 64 rows and a
 // head of 92544 features 674 / 663.  Tiles that do not divide evenly leave CTAs idle: 313 tiles (three on some CTAs, two on most) 66 /
 // 64 at 72 tokens.
-static bool stream_pays(int fmt, int MT, int N)
+static bool stream_pays(int fmt, int MT, int N, int K)
 {
-    const int tiles = N / kBN;
-    return fmt == kDense && MT > 64 && tiles >= 2 * 148 && 10 * tiles >= 8 * 148 * ((tiles + 147) / 148);
+#ifdef B200_GEMM_TOOL
+    return false;  // tool builds measure plans of gemm_kernel
+#else
+    const int    tiles = N / kBN;
+    PlanOverride ov;
+    return fmt == kDense && MT > 64 && tiles >= 2 * 148 && 10 * tiles >= 8 * 148 * ((tiles + 147) / 148)
+           && !lookup_plan(fmt, MT, N, K, &ov);  // a plan: somebody measured gemm_kernel
+#endif
 }
 
 template<class T>
@@ -474,11 +480,11 @@ static bool thin_pays(const b200_linear_desc* d, int m)
     if (!thin_fits(d, m)) {
         return false;
     }
-    PlanOverride ov;
-    const int    N = d->output_dim, K = d->input_dim, nt = (m + 7) / 8;
 #ifdef B200_GEMM_TOOL
     return false;
 #endif
+    PlanOverride ov;
+    const int    N = d->output_dim, K = d->input_dim, nt = (m + 7) / 8;
     return (double)N * K <= kLimit[d->weight_format == kFp8Col ? 2 : d->weight_format][nt - 1] && (nt < 3 || K <= 8192)
            && !lookup_plan(d->weight_format, (m + 15) / 16 * 16, N, K, &ov);  // a plan: somebody measured the tcgen05 kernel
 }
@@ -737,6 +743,14 @@ static int forward_packed(const b200_linear_desc* d, const void* xp, int mt, int
     p.K        = d->input_dim;
     p.MT       = mt;
     p.M        = m;
+    p.epilogue = epilogue;
+    p.out_mode = out_mode;
+    p.ldy      = (int)ldy;
+    p.out_mt   = out_mt;
+    const bool bf = d->dtype == B200_DTYPE_BF16;
+    if (epilogue != 2 && stream_pays(d->weight_format, mt, p.N, p.K)) {
+        return bf ? launch_stream<nv_bfloat16>(p, st) : launch_stream<half>(p, st);
+    }
     const Plan rg = make_plan(d->weight_format, mt, p.N, p.K, epilogue == 2);
     p.splits = rg.splits, p.nw = rg.nw, p.nx = rg.nx, p.na = rg.na;
 #ifdef B200_GEMM_TOOL
@@ -756,11 +770,6 @@ static int forward_packed(const b200_linear_desc* d, const void* xp, int mt, int
         }
         p.residual = nf->residual, p.norm_w = nf->weight, p.norm_eps = nf->eps, p.ssq = nf->ssq, p.norm_ctr = nf->ctr;
     }
-    p.epilogue = epilogue;
-    p.out_mode = out_mode;
-    p.ldy      = (int)ldy;
-    p.out_mt   = out_mt;
-    const bool bf = d->dtype == B200_DTYPE_BF16;
     if (d->weight_format == kU4) {
 #ifdef B200_GEMM_TOOL
         if (rg.tiles == 4) {
@@ -783,9 +792,6 @@ static int forward_packed(const b200_linear_desc* d, const void* xp, int mt, int
             return bf ? launch<nv_bfloat16, kFp8Col, 2>(p, rg.smem, st) : launch<half, kFp8Col, 2>(p, rg.smem, st);
         }
         return bf ? launch<nv_bfloat16, kFp8Col, 1>(p, rg.smem, st) : launch<half, kFp8Col, 1>(p, rg.smem, st);
-    }
-    if (epilogue != 2 && stream_pays(d->weight_format, mt, p.N)) {
-        return bf ? launch_stream<nv_bfloat16>(p, st) : launch_stream<half>(p, st);
     }
     return bf ? launch<nv_bfloat16, kDense, 1>(p, rg.smem, st) : launch<half, kDense, 1>(p, rg.smem, st);
 }
@@ -858,7 +864,20 @@ extern "C" int b200_linear_forward_packed_residual_rmsnorm(const b200_linear_des
                           w.counters, (cudaStream_t)stream, &nf);
 }
 
-// Host-only introspection of the launch plan (tests/test_linear_plan_cpu.py checks its invariants without a GPU).
+extern "C" int b200_linear_kernel(const b200_linear_desc* d, int m, int packed)
+{
+    if (int e = validate_desc(d)) {
+        return e;
+    }
+    if (m <= 0 || m > 128) {
+        return fail(B200_ERR_INVALID_ARG, "linear_kernel: bad arguments");
+    }
+    if (!packed && thin_pays(d, m)) {
+        return B200_LINEAR_FEW_TOKENS;
+    }
+    return stream_pays(d->weight_format, (m + 15) / 16 * 16, d->output_dim, d->input_dim) ? B200_LINEAR_HEAD : B200_LINEAR_TILES;
+}
+
 // Checks one tuned plan against the budgets the kernel relies on (the same ones tests/test_linear_plan_cpu.py asserts).
 static bool plan_entry_ok(const PlanKey& k, const PlanOverride& v)
 {
@@ -923,6 +942,7 @@ extern "C" int b200_linear_load_plans(const char* path)
     return n;
 }
 
+// Host-only introspection of the launch plan (tests/test_linear_plan_cpu.py checks its invariants without a GPU).
 extern "C" int b200_linear_plan(const b200_linear_desc* d, int m, int* out8)
 {
     if (int e = validate_desc(d)) {
