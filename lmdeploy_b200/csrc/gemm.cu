@@ -7,6 +7,7 @@
 #include "linear_thin.cuh"
 
 #include <algorithm>
+#include <climits>
 #include <cstdlib>
 #include <map>
 #include <mutex>
@@ -455,17 +456,22 @@ struct ThinShape {
     int rt, nt, kw;  // 16-feature tiles per warp, 8-token tiles, warps along K
 };
 
-// Which kernel takes m tokens.  The thin kernel's time grows with the weights and the 8-token tiles, the tcgen05 kernel's has a
-// larger constant part (K split and exchange) and hardly looks at m, so the line is a number of weights per format and tile
-// count.  Both sides in us (captured calls back to back, weights of several layers in turn, packed activations for the tcgen05
-// kernel), thin / tcgen05:
-//   u4    1 tile:  25 M 6.4 / 11.8, 59 M 11 / 15.5, 84 M 21.7 / 23.4, 101 M 19.1 / 17.8
-//         2 tiles: 25 M 8.6 / 12.2, 34 M 8.8 / 13.4, 59 M 15.1 / 16.4 (K 4096) and 16.4 / 15.9 (K 14336), 101 M 26 / 18
-//         3 tiles: 25 M 11.0 / 14.3, 34 M 15.4 / 14.7 (K 8192) and 12.3 / 10.7 (K 2048); 15 M 22.9 / 14.8 at K 14336
-//   fp8   1 tile:  59 M 15.4 / 21.8, 84 M 28 / 33, 117 M 28.9 / 29.7;  2 tiles: 59 M 18.3 / 22.0, 84 M 33 / 33
-//         3 tiles: 34 M 14.4 / 18.5, 59 M 25.9 / 23.2
-//   dense 1 tile:  17 M 6.9 / 13.4, 131 M 38 / 43, 190 M 58 / 61, 525 M 151 / 149;  2 tiles: 34 M 17.6 / 18.7, 67 M 31 / 27
-//         3 tiles: 17 M 10.6 / 14.1, 34 M 18.7 / 19.2, 59 M 28 / 26
+// Which kernel takes m tokens.  The thin kernel's time grows with the weights, with the 8-token tiles and with K (a warp's chain of
+// k-groups; few features leave SMs idle beside it), the tcgen05 kernel's has a larger constant part (pack, K split and exchange) and
+// hardly looks at m.  So the lines are weights and K per format and tile count, and beyond one tile also features (K 1024 and N 32768: no
+// split to pay for there).  Both sides in us, b200_linear_forward captured back to back, weights of several layers in turn; thin / pack
+// and tcgen05; f16 and, after ";", bf16 (dense: the same in both):
+//   u4    1 tile:  4096 x 6144 7.3 / 11.4; 7.7 / 11.9, 14336 x 1024 11.3 / 12.8; 13.4 / 13.8, 8192 x 10240 20.6 / 20.2; 22.7 / 22.5, 4096 x 22016 21.1 / 17.3
+//         2 tiles: 4096 x 8192 9.5 / 12.0; 9.9 / 12.4, 8192 x 4096 10.7 / 11.9; 11.0 / 12.4, 4096 x 10240 15.0 / 14.7, 14336 x 1024 15.2 / 12.9
+//         3 tiles: 4096 x 6144 10.9 / 12.5; 11.6 / 13.0, 6144 x 4096 12.4 / 11.4, 8192 x 1024 14.5 / 11.1
+//   fp8   1 tile:  4096 x 14336 15.0 / 21.0; 17.2 / 21.1, 8192 x 10240 25.0 / 31.9; 30.2 / 32.0, 4096 x 22016 25.6 / 29.0; 30.9 / 29.0, 4096 x 32000 28.2 / 29.7
+//         2 tiles: 4096 x 14336 17.0 / 21.2; 19.7 / 21.2, 1024 x 32768 11.4 / 12.5; 12.9 / 12.5, 4096 x 22016 29.6 / 29.1; 35.5 / 29.2
+//         3 tiles: 5120 x 5120 13.2 / 16.9; 15.0 / 16.8, 8192 x 3072 14.9 / 15.3; 16.1 / 15.2, 4096 x 8192 11.9 / 16.4; 13.2 / 16.3, 2048 x
+//         16384 13.0 / 13.4; 14.2 / 13.4
+//   dense 1 tile:  8192 x 1024 9.6 / 10.3, 14336 x 1024 14.9 / 12.2, 14336 x 4096 20.2 / 25.7, 4096 x 32000 40.4 / 43.6, 8192 x 10240 30.6 / 28.4 (12 SMs have two
+//         CTAs, the others one), 4096 x 46336 69 / 61
+//         2 tiles: 4096 x 4096 9.8 / 12.4, 3072 x 6144 12.9 / 13.0, 8192 x 2048 15.1 / 12.5, 5120 x 5120 19.4 / 15.2
+//         3 tiles: 2048 x 4096 6.8 / 10.0, 4096 x 1024 9.5 / 8.7, 4096 x 4096 11.4 / 12.8, 1024 x 16384 10.2 / 9.7
 constexpr int kThinTokens = 24;
 
 static bool thin_fits(const b200_linear_desc* d, int m)
@@ -476,7 +482,15 @@ static bool thin_fits(const b200_linear_desc* d, int m)
 
 static bool thin_pays(const b200_linear_desc* d, int m)
 {
-    constexpr double kLimit[3][3] = {{200e6, 34e6, 34e6}, {88e6, 56e6, 26e6}, {120e6, 80e6, 34e6}};  // dense, u4, fp8
+    struct Line {
+        double weights;
+        int    k, k_per_feature;
+    };
+    constexpr int  kAny        = INT_MAX;
+    constexpr Line kLine[4][3] = {{{136e6, kAny, 8}, {19e6, 4096, 8}, {17e6, 4096, 2}},                 // dense
+                                  {{88e6, kAny, kAny}, {34e6, 8192, kAny}, {26e6, 4096, kAny}},         // u4
+                                  {{132e6, kAny, kAny}, {60e6, kAny, kAny}, {34e6, 6144, kAny}},        // fp8, f16
+                                  {{84e6, kAny, kAny}, {60e6, kAny, kAny}, {34e6, 6144, kAny}}};        // fp8, bf16: three conversions a pair, not one
     if (!thin_fits(d, m)) {
         return false;
     }
@@ -485,12 +499,13 @@ static bool thin_pays(const b200_linear_desc* d, int m)
 #endif
     PlanOverride ov;
     const int    N = d->output_dim, K = d->input_dim, nt = (m + 7) / 8;
-    return (double)N * K <= kLimit[d->weight_format == kFp8Col ? 2 : d->weight_format][nt - 1] && (nt < 3 || K <= 8192)
+    const Line   l = kLine[d->weight_format == kFp8Col ? (d->dtype == B200_DTYPE_BF16 ? 3 : 2) : d->weight_format][nt - 1];
+    return (double)N * K <= l.weights && K <= l.k && (double)K / N <= l.k_per_feature && (nt == 1 || N <= 16384)
            && !lookup_plan(d->weight_format, (m + 15) / 16 * 16, N, K, &ov);  // a plan: somebody measured the tcgen05 kernel
 }
 
 // As few features per CTA as leave all CTAs resident at once (two per SM): more CTAs than that are a second wave with its own
-// start (N 6144: 16 features and 384 CTAs 7.8 us, 32 and 192 CTAs 6.3), fewer leave SMs idle (N 4096: 4.7 and 5.9)
+// start (N 6144: 16 features and 384 CTAs a quarter slower than 32 and 192 CTAs), fewer leave SMs idle (N 4096: 4.7 us and 5.9)
 static ThinShape thin_shape(const b200_linear_desc* d, int m)
 {
     constexpr int kResident = 2 * 148;
@@ -506,7 +521,7 @@ template<class T, int FMT, int RT, int NT>
 static int launch_thin(const Params& p, const ThinParams& shape, cudaStream_t st)
 {
     // k-groups of weights that a warp holds in registers.  The most that fit 128 registers a thread; three CTAs per SM with fewer
-    // in flight and spills: 8.7 us for 6.4 (u4, 4096 x 6144, m 1), 61 for 38 (dense, 4096 x 32000)
+    // in flight and spills were a third slower (u4, 4096 x 6144, m 1), 61 us for 38 (dense, 4096 x 32000)
     constexpr int DEPTH = FMT == kU4 ? 4 / RT : 2 / RT;
     auto          kern  = linear_thin_kernel<T, FMT, RT, NT, DEPTH>;
     static PerDevice configured{};

@@ -14,12 +14,12 @@
 //     there by the lane that needs it.
 // u4 weights become the same T(fma(q, s, t)) as in the tcgen05 kernel, e4m3 weights the same T(weight * scale).
 //
-// Measured (us, captured calls, tcgen05 kernel without its pack launch -> this kernel): u4 4096 x 6144, m 1: 11.8 -> 6.4; 4096 x
-// 4096: 11.0 -> 4.7; 14336 x 4096: 15.5 -> 11.2; 1024 x 1536: 7.0 -> 2.1; fp8 8192 x 7168, m 8: 21.8 -> 16.1; dense 14336 x 4096, m 1:
-// 24.9 -> 18.7.  Small layers are bound by the latency of one launch, large u4 layers by the integer pipe (the unpacking, 57 % busy
-// on the fullest SM) and by how few warps 128 registers leave (4 a scheduler): the tcgen05 kernel takes those.  Weights by
-// bulk copies into shared memory instead (rows of 16..64 features are pieces of 256 to 1024 bytes) were slower, 12.2 us for 6.4;
-// bulk prefetches into L2 ahead of the loads changed 6.3 to 6.2 and 15.6 to 17.5.
+// Measured (us, captured b200_linear_forward, pack and tcgen05 kernel -> this kernel): u4 f16 m 1 4096 x 6144 11.4 -> 7.1, 4096 x 4096
+// 10.0 -> 4.7, 14336 x 4096 14.3 -> 10.9, 1024 x 1536 6.3 -> 2.1; fp8 m 8 8192 x 10240 31.9 -> 25.0; dense m 1 14336 x 4096 24.8 -> 19.9.
+// Small layers are bound by the latency of one launch, large u4 layers by the integer pipe (the unpacking, 57 % busy on the
+// fullest SM) and by how few warps 128 registers leave (4 a scheduler): the tcgen05 kernel takes those.  Weights by bulk copies into
+// shared memory instead (rows of 16..64 features are pieces of 256 to 1024 bytes) took twice as long; bulk prefetches into L2 ahead
+// of the loads changed 6.3 to 6.2 and 15.6 to 17.5.
 #pragma once
 
 #include "gemm.cuh"

@@ -50,3 +50,15 @@ def test_who_reads_packed_activations_or_unaligned_weights(lib, plans):
     assert kernel(lib, 4096, 6144, L.FMT_U4, 1, prepared=(1 << 20) + 16) == TILES
     assert kernel(lib, 4096, 6144, L.FMT_U4, 25) == TILES
     assert kernel(lib, 4096, 6144, 7, 1) == L.ERR_UNSUPPORTED and kernel(lib, 4096, 6144, L.FMT_U4, 129) == L.ERR_INVALID_ARG
+
+
+# both sides of the lines between the kernels: (format, dtype, m, K, N, who was faster there)
+@pytest.mark.parametrize("fmt,dtype,m,K,N,want", [
+    (1, 0, 1, 4096, 6144, FEW), (1, 0, 8, 14336, 1024, FEW), (1, 0, 8, 4096, 22016, TILES), (1, 0, 9, 8192, 4096, FEW), (1, 0, 16, 14336, 1024, TILES),
+    (1, 0, 16, 1024, 32768, TILES), (1, 0, 24, 4096, 6144, FEW), (1, 0, 24, 6144, 4096, TILES), (1, 1, 24, 8192, 1024, TILES),
+    (3, 0, 8, 4096, 32000, FEW), (3, 1, 8, 4096, 22016, TILES), (3, 1, 8, 8192, 10240, FEW), (3, 1, 16, 4096, 14336, FEW), (3, 1, 16, 1024, 32768, TILES),
+    (3, 0, 24, 4096, 8192, FEW), (3, 1, 24, 8192, 1024, TILES),
+    (0, 0, 1, 4096, 32000, FEW), (0, 0, 8, 4096, 46336, TILES), (0, 0, 8, 14336, 1024, TILES), (0, 0, 8, 14336, 4096, FEW), (0, 0, 16, 4096, 4096, FEW), (0, 0, 16, 5120, 5120, TILES),
+    (0, 1, 16, 8192, 1024, TILES), (0, 0, 24, 4096, 4096, FEW), (0, 0, 24, 4096, 1024, TILES), (0, 1, 24, 8192, 2048, TILES)])
+def test_calls_go_to_the_faster_kernel(lib, plans, fmt, dtype, m, K, N, want):
+    assert kernel(lib, K, N, fmt, m, dtype=dtype) == want
