@@ -73,6 +73,14 @@ inline int current_device()
     return dev >= 0 && dev < kMaxDevices ? dev : 0;
 }
 
+// norm.cu: greedy sampling of a model's step by several CTAs per row; scratch of rows * kArgChunks parts, used by one call at a time
+constexpr int kArgChunks = 16;
+struct ArgPart {
+    float value;
+    int   index;
+};
+int argmax_scratch(int* out, const void* logits, int rows, int vocab, int64_t ld, int dtype, void* scratch, void* stream);
+
 #define B200_CUDA_TRY(expr)                                                                                            \
     do {                                                                                                               \
         cudaError_t _e = (expr);                                                                                       \

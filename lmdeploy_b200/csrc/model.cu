@@ -50,6 +50,7 @@ struct b200_model {
     size_t lin_ws_bytes{};
     int*  plan{};
     float* rope_table{};
+    void*  arg_ws{};
     // B200_STEP_TRACE=1: CUDA-event time per operator of every (un-captured) step, printed to stderr -- the analogue of
     // the reference's NVTX ranges around the same calls (utils/nvtx_utils.h:37-50)
     bool trace_on{};
@@ -128,6 +129,7 @@ extern "C" int b200_model_create(b200_model** out, const b200_model_config* c)
     rc = rc ? rc : alloc(&m->lin_ws, lin);
     rc = rc ? rc : alloc((void**)&m->plan, (size_t)(MB + 1) * 4);
     rc = rc ? rc : alloc((void**)&m->rope_table, (size_t)MB * 64 * 8);
+    rc = rc ? rc : alloc(&m->arg_ws, (size_t)MB * kArgChunks * sizeof(ArgPart));
     if (rc) {
         b200_model_destroy(m);
         return rc;
@@ -141,7 +143,7 @@ extern "C" void b200_model_destroy(b200_model* m)
     if (!m) {
         return;
     }
-    void* bufs[] = {m->residual, m->xp, m->qkv, m->attn_xp, m->o, m->act_xp, m->logits, m->attn_ws, m->lin_ws, m->plan, m->rope_table};
+    void* bufs[] = {m->residual, m->xp, m->qkv, m->attn_xp, m->o, m->act_xp, m->logits, m->attn_ws, m->lin_ws, m->plan, m->rope_table, m->arg_ws};
     for (void* p : bufs) {
         if (p) {
             cudaFree(p);
@@ -413,7 +415,7 @@ static int run_step(b200_model* m, const b200_step_inputs* in, int R, bool chunk
             TRY_T(9, b200_comm_argmax_allgather(m->comm, in->out_tokens, m->logits, R, c.vocab, valid, c.dtype, stream));
         }
         else {
-            TRY_T(9, b200_argmax(in->out_tokens, m->logits, R, valid, c.vocab, c.dtype, stream));
+            TRY_T(9, argmax_scratch(in->out_tokens, m->logits, R, valid, c.vocab, c.dtype, m->arg_ws, stream));
         }
     }
     if (in->advance && !chunk) {

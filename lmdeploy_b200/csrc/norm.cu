@@ -116,12 +116,10 @@ __global__ void embedding_kernel(T* out, const T* table, const int* ids, int dim
     }
 }
 
-// greedy: index of the maximum of fp32-cast logits; ties -> smallest index.  Two stages: (rows x kArgChunks) CTAs
-// scan a vocab slice each, then one warp per row merges the partials (deterministic).
-constexpr int kArgChunks  = 16;
+// greedy: index of the maximum of fp32-cast logits; ties -> smallest index.  A model's step takes two stages: (rows x kArgChunks) CTAs scan
+// a vocab slice each into the model's own scratch, then one warp per row merges the slices.  b200_argmax, which has no scratch that
+// belongs to the call, scans each row with one CTA: calls on several streams share nothing.
 constexpr int kArgMaxRows = 1024;
-__device__ float g_arg_val[kArgMaxRows * kArgChunks];
-__device__ int   g_arg_idx[kArgMaxRows * kArgChunks];
 
 __device__ __forceinline__ void arg_better(float& bv, int& bi, float v, int i)
 {
@@ -131,14 +129,15 @@ __device__ __forceinline__ void arg_better(float& bv, int& bi, float v, int i)
     }
 }
 
+// slice blockIdx.y of a row -> part[row][slice], or the row's index where the whole row is one slice
 template<class T>
-__global__ void __launch_bounds__(256) argmax_stage1_kernel(const T* logits, int vocab, int64_t ld)
+__global__ void __launch_bounds__(1024) argmax_stage1_kernel(const T* logits, int vocab, int64_t ld, ArgPart* part, int* out)
 {
     pdl_launch_dependents();
     pdl_wait();
     using Ops    = TypeOps<T>;
-    const int row = blockIdx.x, ch = blockIdx.y;
-    const int per = ((vocab + kArgChunks - 1) / kArgChunks + 7) / 8 * 8;  // slices of whole 16-byte units
+    const int row = blockIdx.x, ch = blockIdx.y, chunks = gridDim.y;
+    const int per = ((vocab + chunks - 1) / chunks + 7) / 8 * 8;  // slices of whole 16-byte units
     const int lo = min(vocab, ch * per), hi = min(vocab, lo + per);
     const T*  lp = logits + (size_t)row * ld;
     float     bv = -INFINITY;
@@ -169,8 +168,8 @@ __global__ void __launch_bounds__(256) argmax_stage1_kernel(const T* logits, int
     for (int i = full + threadIdx.x; i < hi; i += blockDim.x) {
         arg_better(bv, bi, Ops::to_f32(lp[i]), i);
     }
-    __shared__ float s_v[8];
-    __shared__ int   s_i[8];
+    __shared__ float s_v[32];
+    __shared__ int   s_i[32];
 #pragma unroll
     for (int m = 16; m >= 1; m >>= 1) {
         arg_better(bv, bi, __shfl_xor_sync(0xffffffffu, bv, m), __shfl_xor_sync(0xffffffffu, bi, m));
@@ -181,13 +180,17 @@ __global__ void __launch_bounds__(256) argmax_stage1_kernel(const T* logits, int
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        for (int w = 1; w < 8; ++w) arg_better(bv, bi, s_v[w], s_i[w]);
-        g_arg_val[row * kArgChunks + ch] = bv;
-        g_arg_idx[row * kArgChunks + ch] = bi;
+        for (int w = 1; w < (int)blockDim.x / 32; ++w) arg_better(bv, bi, s_v[w], s_i[w]);
+        if (out) {
+            out[row] = bi;
+        }
+        else {
+            part[row * kArgChunks + ch] = ArgPart{bv, bi};
+        }
     }
 }
 
-__global__ void argmax_stage2_kernel(int* out, int rows)
+__global__ void argmax_stage2_kernel(int* out, const ArgPart* part, int rows)
 {
     pdl_launch_dependents();
     pdl_wait();
@@ -195,9 +198,10 @@ __global__ void argmax_stage2_kernel(int* out, int rows)
     if (row >= rows) {
         return;
     }
-    const int lane = threadIdx.x & 31;
-    float     bv   = lane < kArgChunks ? g_arg_val[row * kArgChunks + lane] : -INFINITY;
-    int       bi   = lane < kArgChunks ? g_arg_idx[row * kArgChunks + lane] : 0x7fffffff;
+    const int     lane = threadIdx.x & 31;
+    const ArgPart p    = lane < kArgChunks ? part[row * kArgChunks + lane] : ArgPart{-INFINITY, 0x7fffffff};
+    float         bv   = p.value;
+    int           bi   = p.index;
 #pragma unroll
     for (int m = 16; m >= 1; m >>= 1) {
         arg_better(bv, bi, __shfl_xor_sync(0xffffffffu, bv, m), __shfl_xor_sync(0xffffffffu, bi, m));
@@ -286,22 +290,35 @@ extern "C" int b200_embedding_lookup(void* out, const void* table, const int* to
     return check_launch("embedding_kernel");
 }
 
+static int launch_argmax(const void* logits, int rows, int chunks, int threads, int vocab, int64_t ld, int dtype, ArgPart* part, int* out, cudaStream_t st)
+{
+    const dim3 grid(rows, chunks);
+    if (dtype == B200_DTYPE_F16) {
+        launch_k(argmax_stage1_kernel<half>, grid, dim3(threads), 0, st, (const half*)logits, vocab, ld, part, out);
+    }
+    else {
+        launch_k(argmax_stage1_kernel<nv_bfloat16>, grid, dim3(threads), 0, st, (const nv_bfloat16*)logits, vocab, ld, part, out);
+    }
+    return check_launch("argmax_stage1_kernel");
+}
+
 extern "C" int b200_argmax(int* out, const void* logits, int rows, int vocab, int64_t ld, int dtype, void* stream)
 {
     if (!out || !logits || rows <= 0 || vocab <= 0 || rows > kArgMaxRows) {
         return fail(B200_ERR_INVALID_ARG, "bad argmax arguments (rows <= 1024)");
     }
-    cudaStream_t st = (cudaStream_t)stream;
-    dim3         grid(rows, kArgChunks);
-    if (dtype == B200_DTYPE_F16) {
-        launch_k(argmax_stage1_kernel<half>, dim3(grid), dim3(256), 0, st, (const half*)logits, vocab, ld);
+    return launch_argmax(logits, rows, 1, 1024, vocab, ld, dtype, nullptr, out, (cudaStream_t)stream);
+}
+
+int b200::argmax_scratch(int* out, const void* logits, int rows, int vocab, int64_t ld, int dtype, void* scratch, void* stream)
+{
+    if (!out || !logits || !scratch || rows <= 0 || vocab <= 0) {
+        return fail(B200_ERR_INVALID_ARG, "bad argmax arguments");
     }
-    else {
-        launch_k(argmax_stage1_kernel<nv_bfloat16>, dim3(grid), dim3(256), 0, st, (const nv_bfloat16*)logits, vocab, ld);
-    }
-    if (int e = check_launch("argmax_stage1_kernel")) {
+    ArgPart* part = (ArgPart*)scratch;
+    if (int e = launch_argmax(logits, rows, kArgChunks, 256, vocab, ld, dtype, part, nullptr, (cudaStream_t)stream)) {
         return e;
     }
-    launch_k(argmax_stage2_kernel, dim3((rows + 3) / 4), dim3(128), 0, st, out, rows);
+    launch_k(argmax_stage2_kernel, dim3((rows + 3) / 4), dim3(128), 0, (cudaStream_t)stream, out, (const ArgPart*)part, rows);
     return check_launch("argmax_stage2_kernel");
 }
