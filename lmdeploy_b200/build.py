@@ -75,7 +75,7 @@ def build_hybrid(force=False):
     source or its header is newer; concurrent builders write to a private name and rename."""
     hdr = os.path.join(REPO, "include", "b200_hybrid.h")
     hdir = os.path.dirname(HYBRID_SRC)
-    newest = max([os.path.getmtime(f) for f in (hdr, os.path.join(CSRC, "umma.cuh"), os.path.join(CSRC, "common.cuh"))] + [os.path.getmtime(os.path.join(hdir, f)) for f in os.listdir(hdir) if f.endswith((".cu", ".cuh"))])
+    newest = max([os.path.getmtime(f) for f in (hdr, os.path.join(CSRC, "umma.cuh"), os.path.join(CSRC, "common.cuh"), os.path.join(CSRC, "host_utils.h"))] + [os.path.getmtime(os.path.join(hdir, f)) for f in os.listdir(hdir) if f.endswith((".cu", ".cuh"))])
     if not force and os.path.exists(HYBRID_LIB) and os.path.getmtime(HYBRID_LIB) >= newest:
         return HYBRID_LIB
     os.makedirs(LIBDIR, exist_ok=True)

@@ -19,6 +19,7 @@
 #include <stdint.h>
 #include <atomic>
 #include <initializer_list>
+#include "../host_utils.h"
 #include "../umma.cuh"
 
 namespace b200h {
@@ -1492,23 +1493,6 @@ static bool flash_attention_pays(const b200h_window_args* a)
 
 constexpr int kMaxDevices = 64;
 
-// a launch that may begin before the kernel in front of it has ended (programmatic dependent launch)
-template <class... KArgs, class... Args>
-static cudaError_t launch_early(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, const Args&... args)
-{
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
-}
-
 template <int D, int MAPS, int V>
 static int launch_flash(const FlashArgs& a, cudaStream_t st)
 {
@@ -1525,9 +1509,9 @@ static int launch_flash(const FlashArgs& a, cudaStream_t st)
         if (slot) sms_of[dev].store(sms, std::memory_order_release);
     }
     const int tokens = 128 / (a.heads / a.kv_heads);
-    // each waits for the kernel in front of it on the device
-    if (launch_early(flash_plan_kernel, dim3(1), dim3(1024), 0, st, a, MAPS == 2 ? tokens : 2 * tokens) != cudaSuccess ||
-        launch_early(kernel, dim3(sms), dim3(kFaThreads), FlashShape<D, MAPS, V>::kSmem, st, a) != cudaSuccess)
+    // each may begin before the kernel in front of it has ended, and waits for it on the device
+    if (b200::launch_k(flash_plan_kernel, dim3(1), dim3(1024), 0, st, a, MAPS == 2 ? tokens : 2 * tokens) != cudaSuccess ||
+        b200::launch_k(kernel, dim3(sms), dim3(kFaThreads), FlashShape<D, MAPS, V>::kSmem, st, a) != cudaSuccess)
         return launched("window_attention");
     return 0;
 }
