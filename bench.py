@@ -25,7 +25,7 @@ sys.path.insert(0, ROOT)
 
 # dram__bytes_read.sum + dram__bytes_write.sum per launch of the dominant kernel from the committed ncu --set full
 # capture (profiles/): filled per config once measured
-TRAFFIC_NCU = {"c2": 278094848 + 5309696}   # profiles/r02_attention_ncu.md (r02_attn.ncu-rep): dram read + write per launch
+TRAFFIC_NCU = {"c2": 278094848 + 5309696}   # dram read + write per launch
 
 CONFIGS = {
     # name: (spec, batch, ctx, kv quant policy)
@@ -311,7 +311,7 @@ def measured_peaks():
     if os.path.exists(p):
         d = json.load(open(p))
         return float(d["hbm_gbs"]), "measured (MEASURED_PEAKS.json hbm_gbs)"
-    return 6650.0, "fallback (B200_PROFILING.md)"
+    return 6650.0, "fallback (an earlier measurement)"
 
 
 def _gpu_uuid(torch, local):
@@ -650,7 +650,7 @@ def run_b200(args):
     step_gbs = sb["total"] / (ms_per_step * 1e-3) / 1e9
     roofline = {
         "bound": "hbm", "kernel": "decode_attention_kernel", "achieved": attn["gbs"], "peak": peak, "unit": "GB/s",
-        "frac": attn["gbs"] / peak, "traffic": TRAFFIC_NCU.get(args.config), "traffic_source": "ncu --set full capture of this kernel, profiles/r02_attention_ncu.md (not re-measured in this run)", "peak_source": peak_src,
+        "frac": attn["gbs"] / peak, "traffic": TRAFFIC_NCU.get(args.config), "traffic_source": "ncu --set full capture of this kernel (profiles/, not re-measured in this run)", "peak_source": peak_src,
         "bytes_per_launch": attn["bytes"], "us_per_launch": attn["us"],
         # the whole operator (prologue + main kernel + fix-up), what a caller of b200_decode_attention pays
         "full_op": {"us_per_call": attn_full["us"], "achieved": attn_full["gbs"], "frac": attn_full["gbs"] / peak},

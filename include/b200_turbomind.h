@@ -194,7 +194,9 @@ B200_API int b200_decode_attention_grid(int quant_policy, int dtype);
  *   interleaves or slices output columns (RoPE pair reorder, fused gate|up, TP) expands the checkpoint's blocks
  *   first and hands this format over.  Same arithmetic as format 2.
  * D[m, N] = x[m, K] . dequant(W) (+ bias); u4 dequant is w = fma_T(q, s, -(z*s)_T) exactly as
- * kernels/gemm/transform.h:48-74 / cast.cu:155; accumulation fp32 on tcgen05 tensor cores.
+ * kernels/gemm/transform.h:48-74 / cast.cu:155; products of T weights accumulated in fp32 on tensor cores.  The weights' values do not
+ * depend on m; the order of a sum depends on the kernel that a call runs (b200_linear_kernel), so the same row may come back with
+ * another last bit for another m, for x and y that overlap, or for `prepared` off a 32-byte boundary.
  * epilogue: 0 none; 1 gated SiLU over element-interleaved (gate, up) columns -> [m, N/2]
  *   (kernels/gemm/epilogue.h:158-177).
  * `prepared` is library-owned layout (b200_linear_prepared_bytes bytes); `bias` may be NULL.

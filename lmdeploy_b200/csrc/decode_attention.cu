@@ -576,7 +576,7 @@ static int launch_decode(const b200_attention_params* a)
     }
     // Which parts run inside the main kernel (B200_ATTN_FUSED; debug_flags bits 2 / 3 select per call).  Default 0: the
     // three-kernel form -- prologue kernel, main kernel, fix-up kernel chained by programmatic dependent launch.  Measured
-    // at C2 (profiles/r02_attention_variants.md, ncu per-kernel + CUDA events): the prologue inside the main kernel (bit 0:
+    // at C2 (ncu per kernel and CUDA events): the prologue inside the main kernel (bit 0:
     // RoPE of q in registers, the warp that owns the new token's slot quantises + stores K/V) costs the main kernel +7.2 us
     // (dependent global loads at every segment start / last tile sit on each CTA's critical path) against a 5.9 us kernel
     // that PDL overlaps; the fix-up inside (bit 1) costs +6.2 us (an acq_rel atomic round trip + two dependent L2 passes per
@@ -605,7 +605,7 @@ static int launch_decode(const b200_attention_params* a)
     // prologue kernel, and is pointless without it.  B200_ATTN_EARLY=0 turns it off (A/B measurements).
     static const bool env_early = [] {
         const char* e = getenv("B200_ATTN_EARLY");
-        return !(e && *e == '0');  // measured: 4.148 -> 4.101 ms per C2 step (profiles/r02_attention_variants.md)
+        return !(e && *e == '0');  // measured: 4.148 -> 4.101 ms per C2 step
     }();
     const bool run_prologue = !(want & 1) && !(a->debug_flags & 1);
     const int  early        = env_early && a->plan != nullptr && run_prologue ? 1 : 0;

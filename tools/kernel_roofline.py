@@ -12,7 +12,7 @@ sys.path.insert(0, os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
 from lmdeploy_b200.turbomind.specs import SPECS  # noqa: E402
 
 CONFIGS = {"c2": ("internlm2-7b", 64, 2048, 8), "c3": ("llama3-8b", 128, 4096, 4), "c4": ("internlm2-20b", 64, 2048, 0)}
-# measured on B200 (profiles/r01b_*.md; GEMMs graph-timed by tools/gemm_trace.cu, attention by bench.py)
+# measured on B200 (GEMMs graph-timed by tools/gemm_trace.cu, attention by bench.py)
 MEASURED_US = {"c2": {"qkv": 12.8, "wo": 10.6, "w1w3": 22.6, "w2": 15.9, "attention": 56.6, "lm_head": 116.0,
                       "kv prologue": 5.7, "attention fix-up": 5.5, "residual+rmsnorm x2": 8.0}}
 
