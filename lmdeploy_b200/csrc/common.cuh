@@ -171,6 +171,16 @@ B200_DEVICE uint32_t lds32(uint32_t addr)
     return v;
 }
 
+// 16 bytes from global into shared memory, past the L1; in place after cp_async_wait_all
+B200_DEVICE void cp_async16(uint32_t dst, const void* src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+B200_DEVICE void cp_async_wait_all()
+{
+    asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
 // 32 bytes to global memory: in one write (a whole sector) where the address is a multiple of 32, else in two
 B200_DEVICE void store_words8(void* p, const uint32_t (&v)[8], bool wide)
 {

@@ -658,11 +658,11 @@ static int launch_decode(const b200_attention_params* a)
         return 0;
     }
     dim3 rgrid(a->num_kv_heads, a->batch_size);
-    const int per = kHeadDim / 4 * (a->num_heads / a->num_kv_heads);  // four dims per thread
-    if (merge_in_runs(p, grid)) {
-        launch_k(decode_reduce_groups_kernel<T>, dim3(rgrid), dim3(per * kReduceGroups), 0, st, p, grid);
+    if (few_segments(p, grid)) {
+        launch_k(decode_reduce_heads_kernel<T>, dim3(a->num_heads, a->batch_size), dim3(kHeadDim), 0, st, p, grid);
     }
     else {
+        const int per = kHeadDim / 4 * (a->num_heads / a->num_kv_heads);  // four dims per thread
         launch_k(decode_reduce_kernel<T>, dim3(rgrid), dim3(per), 0, st, p, grid);
     }
     return check_launch("decode_reduce_kernel");

@@ -886,66 +886,12 @@ B200_DEVICE SegCtas segment_ctas(const KernelParams& p, int b, int h, int grid_m
     return s;
 }
 
-// Few segments have many pieces each (four or more on average).  Their merge takes the pieces in kReduceGroups runs -- by one group of
-// threads per run in decode_reduce_groups_kernel, one run after the other where the main kernel merges itself -- and then the runs in
-// order, with the same roundings in both.
-constexpr int kReduceGroups = 4;
-__host__ B200_DEVICE bool merge_in_runs(const KernelParams& p, int grid_main)
-{
-    return grid_main >= 4 * p.num_kv_heads * p.batch;
-}
-
-struct MergeRun {
-    float  m, l;  // maximum and sum of weights relative to it
-    float4 o;
-};
-
 B200_DEVICE int merge_slot(const SegCtas& sg, int grid_main, int k)
 {
     if (sg.sparse) {
         return 2 * (int)(((sg.s0 + k + 1) * grid_main - 1) / sg.total);  // one unit per CTA: always its first slot
     }
     return 2 * (sg.cf + k) + (k == 0 ? sg.first_slot : 0);
-}
-
-B200_DEVICE void merge_into(MergeRun& r, float w, float l, const float4& o)
-{
-    r.l   = fmaf(w, l, r.l);
-    r.o.x = fmaf(w, o.x, r.o.x), r.o.y = fmaf(w, o.y, r.o.y), r.o.z = fmaf(w, o.z, r.o.z), r.o.w = fmaf(w, o.w, r.o.w);
-}
-
-// run `grp` of a segment's pieces: four dims from i on, of head hd; maximum and sum in one read of four pieces at a time
-B200_DEVICE MergeRun merge_run(const KernelParams& p, const SegCtas& sg, int grid_main, int grp, int hd, int i)
-{
-    constexpr int kBatch = 4;
-    const float   c  = p.qk_scale;
-    const int     k1 = sg.n * (grp + 1) / kReduceGroups;
-    MergeRun      r{-INFINITY, 0.f, make_float4(0.f, 0.f, 0.f, 0.f)};
-    for (int k0 = sg.n * grp / kReduceGroups; k0 < k1; k0 += kBatch) {
-        float2 ml[kBatch];
-        float4 o[kBatch];
-#pragma unroll
-        for (int k = 0; k < kBatch; ++k) {
-            ml[k] = make_float2(-INFINITY, 0.f);
-            o[k]  = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (k0 + k < k1) {
-                const int slot = merge_slot(sg, grid_main, k0 + k);
-                ml[k] = __ldcg(reinterpret_cast<const float2*>(&p.partial_ML[((size_t)slot * kMaxGroup + hd) * 2]));
-                o[k]  = __ldcg(reinterpret_cast<const float4*>(&p.partial_O[(size_t)slot * kMaxGroup * kHeadDim + i]));
-            }
-        }
-        float top = r.m;
-#pragma unroll
-        for (int k = 0; k < kBatch; ++k) top = fmaxf(top, ml[k].x);
-        const float a = r.m == -INFINITY ? 0.f : exp2_approx((r.m - top) * c);
-        r.l *= a, r.o.x *= a, r.o.y *= a, r.o.z *= a, r.o.w *= a;
-        r.m = top;
-#pragma unroll
-        for (int k = 0; k < kBatch; ++k) {
-            merge_into(r, ml[k].x == -INFINITY ? 0.f : exp2_approx((ml[k].x - top) * c), ml[k].y, o[k]);
-        }
-    }
-    return r;
 }
 
 template<class T>
@@ -960,26 +906,11 @@ B200_DEVICE void merge_store(const KernelParams& p, int b, int h, int i, const f
     *reinterpret_cast<uint2*>(dst) = v;
 }
 
-template<class T, class GetRun>
-B200_DEVICE void merge_runs(const KernelParams& p, int b, int h, int i, GetRun get)
-{
-    float m = -INFINITY;
-#pragma unroll
-    for (int q = 0; q < kReduceGroups; ++q) m = fmaxf(m, get(q).m);
-    MergeRun r{m, 0.f, make_float4(0.f, 0.f, 0.f, 0.f)};
-#pragma unroll
-    for (int q = 0; q < kReduceGroups; ++q) {
-        const MergeRun x = get(q);
-        merge_into(r, x.m == -INFINITY ? 0.f : exp2_approx((x.m - m) * p.qk_scale), x.l, x.o);
-    }
-    merge_store<T>(p, b, h, i, r.o, r.l);
-}
-
 // Merge of the partials of one segment.  Same math as attention::reduce (reduce.cu:90-153): O = sum_k w_k O_k / sum_k w_k L_k,
 // w_k = exp2((M_k - M) * c), pieces visited in ascending CTA order whoever runs the merge (deterministic).  Loads bypass L1
 // (ld.global.cg): the partials may have been written by other SMs during this very kernel.
 template<class T>
-__device__ __noinline__ void merge_in_order(const KernelParams& p, int b, int h, const SegCtas& sg, int grid_main, int tid,
+__device__ __noinline__ void merge_segment(const KernelParams& p, int b, int h, const SegCtas& sg, int grid_main, int tid,
                                            int nthreads)
 {
     const int   G = p.num_heads / p.num_kv_heads;
@@ -1033,21 +964,6 @@ __device__ __noinline__ void merge_in_order(const KernelParams& p, int b, int h,
         }
         merge_store<T>(p, b, h, i, acc, l);
     }
-}
-
-template<class T>
-__device__ __noinline__ void merge_segment(const KernelParams& p, int b, int h, const SegCtas& sg, int grid_main, int tid, int nthreads)
-{
-    const int G = p.num_heads / p.num_kv_heads;
-    if (merge_in_runs(p, grid_main)) {
-        for (int i4 = tid; i4 < G * kHeadDim / 4; i4 += nthreads) {
-            MergeRun run[kReduceGroups];
-            for (int q = 0; q < kReduceGroups; ++q) run[q] = merge_run(p, sg, grid_main, q, i4 * 4 / kHeadDim, i4 * 4);
-            merge_runs<T>(p, b, h, i4 * 4, [&](int q) { return run[q]; });
-        }
-        return;
-    }
-    merge_in_order<T>(p, b, h, sg, grid_main, tid, nthreads);
 }
 
 B200_DEVICE int atom_add_acq_rel_gpu(int* p, int v)
@@ -1498,40 +1414,91 @@ __global__ void __launch_bounds__(256) decode_reduce_kernel(const __grid_constan
     if (s_seg.n <= 1) {
         return;  // written directly by the main kernel
     }
-    merge_in_order<T>(p, b, h, s_seg, grid_main, threadIdx.x, blockDim.x);
+    merge_segment<T>(p, b, h, s_seg, grid_main, threadIdx.x, blockDim.x);
 }
 
-// The same for a few long sequences, whose pieces merge_segment's threads would read four at a time, each batch behind the one before: a
-// group of threads per run.  Three sequences of 37 - 7001 bf16 tokens, 48 / 8 heads, whole operator: 24.4 -> 18.0 us; one of 4096
-// int8 tokens, 32 / 8 heads: 31.2 -> 13.0 us.
-template<class T>
-__global__ void __launch_bounds__(kReduceGroups * 256) decode_reduce_groups_kernel(const __grid_constant__ KernelParams p, int grid_main)
+// The same for few segments, which have many pieces each (four or more on average): merge_segment's threads would read eight of them at a
+// time, each batch behind the one before, on one SM per segment.  Here a CTA takes one query head; its warps copy the pieces of it into
+// shared memory, up to 64 at once, and a thread sums one dimension in the same order with the same roundings, so no output depends on
+// which of the two kernels ran.
+// us, whole operator, captured calls, decode_reduce_kernel -> this: three sequences of 37 - 7001 bf16 tokens, 48 / 8 heads, 26.4 -> 19.7; one of 4096
+// int8 tokens, 32 / 8 heads, 32.6 -> 12.6; one of 8000 int4 tokens, 8 / 2 heads, 63 -> 16.2; at the line twelve of 700 - 1500 int8 tokens, 32 / 8 heads,
+// 19.0 -> 16.4, and 37 of 5000 - 5496, 8 / 2 heads, 31.0 -> 27.2.  (All loads of a thread in registers instead, 32 or 64 at once: 21.0 for 19.7.)
+constexpr int kReduceBatch = 64;
+__host__ B200_DEVICE bool few_segments(const KernelParams& p, int grid_main)
 {
+    return grid_main >= 4 * p.num_kv_heads * p.batch;
+}
+
+template<class T>
+__global__ void __launch_bounds__(kHeadDim) decode_reduce_heads_kernel(const __grid_constant__ KernelParams p, int grid_main)
+{
+    using Ops = TypeOps<T>;
+    __shared__ __align__(16) float s_o[kReduceBatch][kHeadDim];
+    __shared__ int    s_slot[kReduceBatch];  // where the pieces lie
+    __shared__ float2 s_wl[kReduceBatch];    // their weight and sum
+    __shared__ float  s_top[kHeadDim / 32];
     pdl_launch_dependents();
     pdl_wait();
-    const int b = blockIdx.y, h = blockIdx.x;
+    const int G = p.num_heads / p.num_kv_heads, b = blockIdx.y, h = blockIdx.x / G, hd = blockIdx.x - h * G, d = threadIdx.x;
     if (p.tile_prefix[b + 1] == p.tile_prefix[b]) {
         return;
     }
-    __shared__ SegCtas s_seg;
-    if (threadIdx.x == 0) {
-        s_seg = segment_ctas(p, b, h, grid_main);
-    }
-    __syncthreads();
-    if (s_seg.n <= 1) {
+    const SegCtas sg = segment_ctas(p, b, h, grid_main);
+    if (sg.n <= 1) {
         return;  // written directly by the main kernel
     }
-    __shared__ float4 s_o[kReduceGroups][kMaxGroup * kHeadDim / 4];
-    __shared__ float2 s_ml[kReduceGroups][kMaxGroup * kHeadDim / 4];
-    const int per = p.num_heads / p.num_kv_heads * kHeadDim / 4;
-    const int grp = threadIdx.x / per, i4 = threadIdx.x - grp * per, i = i4 * 4;
-    MergeRun  r   = merge_run(p, s_seg, grid_main, grp, i / kHeadDim, i);
-    s_o[grp][i4]  = r.o;
-    s_ml[grp][i4] = make_float2(r.m, r.l);
-    __syncthreads();
-    if (grp == 0) {
-        merge_runs<T>(p, b, h, i, [&](int q) { return MergeRun{s_ml[q][i4].x, s_ml[q][i4].y, s_o[q][i4]}; });
+    auto read = [&](int slot) { return __ldcg(reinterpret_cast<const float2*>(&p.partial_ML[((size_t)slot * kMaxGroup + hd) * 2])); };
+    // pieces k1 .. k1 + kReduceBatch - 1: their slots, and copies of their values on the way
+    auto fetch = [&](int k1) {
+        const int n = min(sg.n - k1, kReduceBatch);
+        if (d < n) {
+            s_slot[d] = merge_slot(sg, grid_main, k1 + d);
+        }
+        __syncthreads();
+        for (int k = d >> 5; k < n; k += kHeadDim / 32) {
+            const int i = (d & 31) * 4;
+            cp_async16(smem_u32(&s_o[k][i]), &p.partial_O[((size_t)s_slot[k] * kMaxGroup + hd) * kHeadDim + i]);
+        }
+        return n;
+    };
+    int    n  = fetch(0);
+    float2 ml = d < n ? read(s_slot[d]) : make_float2(-INFINITY, 0.f);
+    float  m  = ml.x;
+    for (int k = kReduceBatch + d; k < sg.n; k += kHeadDim) m = fmaxf(m, read(merge_slot(sg, grid_main, k)).x);
+#pragma unroll
+    for (int x = 16; x >= 1; x >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, x));
+    if ((d & 31) == 0) {
+        s_top[d >> 5] = m;
     }
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < kHeadDim / 32; ++w) m = fmaxf(m, s_top[w]);
+    float acc = 0.f, l = 0.f;
+    for (int k1 = 0;;) {
+        if (d < n) {
+            s_wl[d] = make_float2(ml.x == -INFINITY ? 0.f : exp2_approx((ml.x - m) * p.qk_scale), ml.y);
+        }
+        cp_async_wait_all();
+        __syncthreads();
+#pragma unroll 4
+        for (int k = 0; k < n; ++k) {
+            const float2 wl = s_wl[k];
+            l += wl.x * wl.y;
+            acc += wl.x * s_o[k][d];
+        }
+        if ((k1 += kReduceBatch) >= sg.n) {
+            break;
+        }
+        __syncthreads();  // read by everyone
+        n = fetch(k1);
+        if (d < n) {
+            ml = read(s_slot[d]);
+        }
+    }
+    const int col = blockIdx.x * kHeadDim + d;
+    T*        out = reinterpret_cast<T*>(p.out);
+    out[p.out_mt > 0 ? ((size_t)(col >> 3) * p.out_mt + b) * 8 + (col & 7) : (size_t)b * p.out_stride + col] = Ops::from_f32(acc / l);
 }
 
 }  // namespace attn

@@ -1,5 +1,5 @@
-"""Decode attention of a few sequences: their pieces are merged in four runs (decode_reduce_groups_kernel).  Lengths that leave a run empty,
-one piece, more pieces than runs times the batch of reads, sequences without keys beside long ones; against the numpy oracle."""
+"""Decode attention of a few sequences, whose pieces a CTA per query head merges (decode_reduce_heads_kernel): one piece, a few, sequences without
+keys beside long ones; against the numpy oracle."""
 import numpy as np
 import pytest
 
