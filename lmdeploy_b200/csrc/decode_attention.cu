@@ -659,12 +659,9 @@ static int launch_decode(const b200_attention_params* a)
     }
     dim3 rgrid(a->num_kv_heads, a->batch_size);
     if (few_segments(p, grid)) {
-        launch_k(decode_reduce_heads_kernel<T>, dim3(a->num_heads, a->batch_size), dim3(kHeadDim), 0, st, p, grid);
+        return launch_reduce_heads(std::is_same<T, nv_bfloat16>::value, p, grid, st);
     }
-    else {
-        const int per = kHeadDim / 4 * (a->num_heads / a->num_kv_heads);  // four dims per thread
-        launch_k(decode_reduce_kernel<T>, dim3(rgrid), dim3(per), 0, st, p, grid);
-    }
+    launch_k(decode_reduce_kernel<T>, dim3(rgrid), dim3(kHeadDim / 4 * (a->num_heads / a->num_kv_heads)), 0, st, p, grid);  // four dims per thread
     return check_launch("decode_reduce_kernel");
 }
 

@@ -158,7 +158,7 @@ __device__ __forceinline__ void rope_rotate4(T (&x)[4], const float2 (&cs)[2], c
 }
 
 // out of line: the exact-math variant drags double-precision sincos (and its stack frame) into whoever inlines it
-__device__ __noinline__ float2 rope_cos_sin_call(const RopeConst& r, int idx, int pos)
+inline __device__ __noinline__ float2 rope_cos_sin_call(const RopeConst& r, int idx, int pos)
 {
     return rope_cos_sin(r, idx, pos);
 }
@@ -886,26 +886,6 @@ B200_DEVICE SegCtas segment_ctas(const KernelParams& p, int b, int h, int grid_m
     return s;
 }
 
-B200_DEVICE int merge_slot(const SegCtas& sg, int grid_main, int k)
-{
-    if (sg.sparse) {
-        return 2 * (int)(((sg.s0 + k + 1) * grid_main - 1) / sg.total);  // one unit per CTA: always its first slot
-    }
-    return 2 * (sg.cf + k) + (k == 0 ? sg.first_slot : 0);
-}
-
-template<class T>
-B200_DEVICE void merge_store(const KernelParams& p, int b, int h, int i, const float4& acc, float l)
-{
-    using Ops     = TypeOps<T>;
-    const int col = h * (p.num_heads / p.num_kv_heads) * kHeadDim + i;
-    T*        dst = reinterpret_cast<T*>(p.out) + (p.out_mt > 0 ? ((size_t)(col >> 3) * p.out_mt + b) * 8 + (col & 7) : (size_t)b * p.out_stride + col);
-    uint2     v;
-    v.x = Ops::pack2(acc.x / l, acc.y / l);
-    v.y = Ops::pack2(acc.z / l, acc.w / l);
-    *reinterpret_cast<uint2*>(dst) = v;
-}
-
 // Merge of the partials of one segment.  Same math as attention::reduce (reduce.cu:90-153): O = sum_k w_k O_k / sum_k w_k L_k,
 // w_k = exp2((M_k - M) * c), pieces visited in ascending CTA order whoever runs the merge (deterministic).  Loads bypass L1
 // (ld.global.cg): the partials may have been written by other SMs during this very kernel.
@@ -913,15 +893,23 @@ template<class T>
 __device__ __noinline__ void merge_segment(const KernelParams& p, int b, int h, const SegCtas& sg, int grid_main, int tid,
                                            int nthreads)
 {
+    using Ops     = TypeOps<T>;
     const int   G = p.num_heads / p.num_kv_heads;
     const float c = p.qk_scale;
-    auto slot_of  = [&](int k) { return merge_slot(sg, grid_main, k); };
+    auto slot_of  = [&](int k) {
+        if (sg.sparse) {
+            return 2 * (int)(((sg.s0 + k + 1) * grid_main - 1) / sg.total);  // one unit per CTA: always its first slot
+        }
+        const int cta = sg.cf + k;
+        return 2 * cta + (k == 0 ? sg.first_slot : 0);
+    };
     // thread -> 4 consecutive dims of one head (float4 partial loads)
     for (int i4 = tid; i4 < G * kHeadDim / 4; i4 += nthreads) {
         const int i  = i4 * 4;
         const int hd = i / kHeadDim;
         float     m  = -INFINITY;
-        // kBatch pieces' loads in flight, summed in order
+        // kBatch pieces' loads in flight, summed in order (one dependent load after the other: 43 us for 27, 3 sequences of 37 - 7001 bf16
+        // tokens, 48 / 8 heads, whole operator)
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
         float  l   = 0.f;
         auto   sum = [&](auto batch) {
@@ -962,7 +950,13 @@ __device__ __noinline__ void merge_segment(const KernelParams& p, int b, int h, 
         else {
             sum(std::integral_constant<int, 8>{});
         }
-        merge_store<T>(p, b, h, i, acc, l);
+        const int col = h * G * kHeadDim + i;
+        T*        dst = reinterpret_cast<T*>(p.out)
+                 + (p.out_mt > 0 ? ((size_t)(col >> 3) * p.out_mt + b) * 8 + (col & 7) : (size_t)b * p.out_stride + col);
+        uint2 v;
+        v.x = Ops::pack2(acc.x / l, acc.y / l);
+        v.y = Ops::pack2(acc.z / l, acc.w / l);
+        *reinterpret_cast<uint2*>(dst) = v;
     }
 }
 
@@ -1417,89 +1411,9 @@ __global__ void __launch_bounds__(256) decode_reduce_kernel(const __grid_constan
     merge_segment<T>(p, b, h, s_seg, grid_main, threadIdx.x, blockDim.x);
 }
 
-// The same for few segments, which have many pieces each (four or more on average): merge_segment's threads would read eight of them at a
-// time, each batch behind the one before, on one SM per segment.  Here a CTA takes one query head; its warps copy the pieces of it into
-// shared memory, up to 64 at once, and a thread sums one dimension in the same order with the same roundings, so no output depends on
-// which of the two kernels ran.
-// us, whole operator, captured calls, decode_reduce_kernel -> this: three sequences of 37 - 7001 bf16 tokens, 48 / 8 heads, 26.4 -> 19.7; one of 4096
-// int8 tokens, 32 / 8 heads, 32.6 -> 12.6; one of 8000 int4 tokens, 8 / 2 heads, 63 -> 16.2; at the line twelve of 700 - 1500 int8 tokens, 32 / 8 heads,
-// 19.0 -> 16.4, and 37 of 5000 - 5496, 8 / 2 heads, 31.0 -> 27.2.  (All loads of a thread in registers instead, 32 or 64 at once: 21.0 for 19.7.)
-constexpr int kReduceBatch = 64;
-__host__ B200_DEVICE bool few_segments(const KernelParams& p, int grid_main)
-{
-    return grid_main >= 4 * p.num_kv_heads * p.batch;
-}
-
-template<class T>
-__global__ void __launch_bounds__(kHeadDim) decode_reduce_heads_kernel(const __grid_constant__ KernelParams p, int grid_main)
-{
-    using Ops = TypeOps<T>;
-    __shared__ __align__(16) float s_o[kReduceBatch][kHeadDim];
-    __shared__ int    s_slot[kReduceBatch];  // where the pieces lie
-    __shared__ float2 s_wl[kReduceBatch];    // their weight and sum
-    __shared__ float  s_top[kHeadDim / 32];
-    pdl_launch_dependents();
-    pdl_wait();
-    const int G = p.num_heads / p.num_kv_heads, b = blockIdx.y, h = blockIdx.x / G, hd = blockIdx.x - h * G, d = threadIdx.x;
-    if (p.tile_prefix[b + 1] == p.tile_prefix[b]) {
-        return;
-    }
-    const SegCtas sg = segment_ctas(p, b, h, grid_main);
-    if (sg.n <= 1) {
-        return;  // written directly by the main kernel
-    }
-    auto read = [&](int slot) { return __ldcg(reinterpret_cast<const float2*>(&p.partial_ML[((size_t)slot * kMaxGroup + hd) * 2])); };
-    // pieces k1 .. k1 + kReduceBatch - 1: their slots, and copies of their values on the way
-    auto fetch = [&](int k1) {
-        const int n = min(sg.n - k1, kReduceBatch);
-        if (d < n) {
-            s_slot[d] = merge_slot(sg, grid_main, k1 + d);
-        }
-        __syncthreads();
-        for (int k = d >> 5; k < n; k += kHeadDim / 32) {
-            const int i = (d & 31) * 4;
-            cp_async16(smem_u32(&s_o[k][i]), &p.partial_O[((size_t)s_slot[k] * kMaxGroup + hd) * kHeadDim + i]);
-        }
-        return n;
-    };
-    int    n  = fetch(0);
-    float2 ml = d < n ? read(s_slot[d]) : make_float2(-INFINITY, 0.f);
-    float  m  = ml.x;
-    for (int k = kReduceBatch + d; k < sg.n; k += kHeadDim) m = fmaxf(m, read(merge_slot(sg, grid_main, k)).x);
-#pragma unroll
-    for (int x = 16; x >= 1; x >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, x));
-    if ((d & 31) == 0) {
-        s_top[d >> 5] = m;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int w = 0; w < kHeadDim / 32; ++w) m = fmaxf(m, s_top[w]);
-    float acc = 0.f, l = 0.f;
-    for (int k1 = 0;;) {
-        if (d < n) {
-            s_wl[d] = make_float2(ml.x == -INFINITY ? 0.f : exp2_approx((ml.x - m) * p.qk_scale), ml.y);
-        }
-        cp_async_wait_all();
-        __syncthreads();
-#pragma unroll 4
-        for (int k = 0; k < n; ++k) {
-            const float2 wl = s_wl[k];
-            l += wl.x * wl.y;
-            acc += wl.x * s_o[k][d];
-        }
-        if ((k1 += kReduceBatch) >= sg.n) {
-            break;
-        }
-        __syncthreads();  // read by everyone
-        n = fetch(k1);
-        if (d < n) {
-            ml = read(s_slot[d]);
-        }
-    }
-    const int col = blockIdx.x * kHeadDim + d;
-    T*        out = reinterpret_cast<T*>(p.out);
-    out[p.out_mt > 0 ? ((size_t)(col >> 3) * p.out_mt + b) * 8 + (col & 7) : (size_t)b * p.out_stride + col] = Ops::from_f32(acc / l);
-}
+// decode_merge.cu: the fix-up of few segments with many pieces each, when it is the better one and its launch
+bool few_segments(const KernelParams& p, int grid_main);
+int  launch_reduce_heads(bool bf16, const KernelParams& p, int grid_main, cudaStream_t st);
 
 }  // namespace attn
 }  // namespace b200
