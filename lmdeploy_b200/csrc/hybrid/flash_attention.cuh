@@ -20,9 +20,10 @@
 // every role, and beside 224 KB of shared memory the L1 is too small to hold what spills.  So a row's scores are read from tensor
 // memory twice, 32 at a time, instead of being held.
 // Measured (B200, 4 x 1024 rows of causal attention, 16 / 8 heads of 128, with the projection): 2034 us by the two passes, which
-// multiply on the float units; 155 us with 16-byte asynchronous copies from seven loaders of 64 registers (10.2 k cycles per 128 keys: the
-// copies enter shared memory at one per cycle and SM and contend with the products' operands), 129 us now (5.5 k cycles per 128 keys,
-// of which the products take 4.1 k; a piece's start 10 k, its output 6 k).  500 - 1000 rows behind 700 keys, 32 / 8 heads: 288 -> 213 us.
+// multiply on the float units; 158 us with 16-byte asynchronous copies from seven loaders of 64 registers (10.2 k cycles per 128 keys: the
+// copies enter shared memory at one per cycle and SM and contend with the products' operands), 125 us now (5.5 k cycles per 128 keys,
+// of which the products take 4.1 k; a piece's start 10 k, its output 6 k); in runs of a second, at lower clocks, 130 - 133.  Three
+// sequences of 500 - 1000 rows behind 700 keys, 32 / 8 heads, width 4096: 405 -> 301 us.
 
 using b200::smem_u32;
 

@@ -10,7 +10,9 @@
 //   * a stage is half a k-group (64 k's: 16 KB of weights per tile, MT * 128 bytes of X), its copies issued by one lane each.
 //     (Pieces of 2 KB, which would let one multiplication take all 256 features, are issue-bound: 203 us for 176 below.)
 // Measured, 128 tokens, f16 4096 x 128256: 195 -> 176 us in a short run; in a long one the card's power limit (990 W, SM clock down
-// to 0.9 GHz) bounds it, 231 -> 213.
+// to 0.9 GHz) bounds it, 231 -> 213.  First calls on freshly prepared weights, both kernels in one process: after a second of idling 202 -> 182; behind
+// 1.5 s of repeated calls of this kernel 285 -> 235, of gemm_kernel 238 -> 198 (the card is still at the lower clocks; the preparation, unchanged,
+// takes 3.7, 5.3 and 4.5 ms there).  Pairs of tiles dealt out in turn, so that all CTAs walk one window, made no difference to either.
 #pragma once
 
 #include "gemm.cuh"

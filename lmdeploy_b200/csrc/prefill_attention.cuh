@@ -27,9 +27,10 @@
 // 3.47e-4 / 2.70e-3 (and 178 instead of 181 us); one CTA per 128 rows with a maximum per 64 keys had 3.43e-4 / 2.67e-3.
 // Measured (B200, whole operator; before = one CTA per 128 rows, 64-key tiles, the phases one after another): 2 x 64 tokens over
 // 700-1800 int8 keys, 32 / 8 heads: 160 -> 37 us, 35 with queries read and outputs written in whole lines and sectors; prompts of 2048,
-// 1190 and 2048 tokens, f16 pages: 465 -> 181 us (446 TFLOP/s), 166 so.
-// A 256 x 128 step takes about 5 k cycles where the tensor pipe needs 2.0 k and the exponentials 2.0 k: T pages wait for their
-// copies (16-byte pieces through the load/store unit move about 17 bytes a cycle), quantised ones for the conversion.
+// 1190 and 2048 tokens, f16 pages: 465 -> 181 us (446 TFLOP/s), 169 so.  (Short runs; in runs of a second the card's power limit brings the clocks
+// down: 190 and 178 - 182.)
+// A 256 x 128 step takes about 5 k cycles where the tensor pipe needs 2.0 k and the exponentials 2.0 k: the chain scores - maximum - weights of
+// a tile bounds it beside them.  T pages by way of registers instead of 16-byte asynchronous copies changed nothing.
 #pragma once
 
 #include "common.cuh"
