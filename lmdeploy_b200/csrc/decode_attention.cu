@@ -473,7 +473,7 @@ __global__ void __launch_bounds__(128) prefill_prologue_kernel(const ProloguePar
 template<int KVBITS>
 constexpr int stages_for()
 {
-    return KVBITS == 4 ? 6 : 3;  // int4: 4, 5, 6 and 7 measure 140.5, 139, 138.6 and 138.8 us (128 x 4096)
+    return KVBITS == 4 ? 6 : 3;  // int4: 4, 5, 6 and 7 measure 147.0, 144.4, 144.1 and 143.8 us (128 x 4096), 49.6, 49.2, 49.2 and 49.6 (64 x 2048)
 }
 
 template<class T, int KVBITS>

@@ -18,8 +18,8 @@
 // Shared-memory tile layout: rows (tokens) of 128 / 256 bytes are copied in groups of 16 with 32 bytes of padding between
 // groups; together with the slot->token permutation below this makes every LDS of the fragment loads
 // bank-conflict free without TMA swizzling (pages are addressed by pointer, so no tensor map exists for them).
-// Rows of 64 bytes (int4) lie without padding, as in the page: a tile is one copy (and one of its parameters); the
-// loads of V then take two passes each.
+// Rows of 64 bytes (int4) are copied in two groups of 32 with 64 bytes between them, so that a tile takes few copies: the
+// loads of K are free of conflicts, those of V take two passes each.
 #pragma once
 
 #include "common.cuh"
@@ -29,7 +29,6 @@ namespace attn {
 
 constexpr int kHeadDim       = 128;
 constexpr int kTile          = 64;  // tokens per pipeline stage
-constexpr int kGroupRows     = 16;
 constexpr int kConsumerWarps = 4;
 constexpr int kThreads       = (kConsumerWarps + 1) * 32;
 constexpr int kMaxGroup      = 8;  // q heads per kv head handled by one CTA (mma N)
@@ -38,9 +37,11 @@ template<int KVBITS>
 struct TileCfg {
     static constexpr bool kQuant     = KVBITS != 16;
     static constexpr int  kRowBytes  = kHeadDim * KVBITS / 8;
-    static constexpr int  kGroupPad  = KVBITS == 4 ? 0 : 32;
+    static constexpr int  kGroupRows = KVBITS == 4 ? 32 : 16;
+    static constexpr int  kGroupPad  = KVBITS == 4 ? 64 : 32;
     static constexpr int  kGroupSize = kGroupRows * kRowBytes + kGroupPad;
-    static constexpr int  kTileBytes = (kTile / kGroupRows) * kGroupSize;
+    // int4: V begins where K ends (no padding behind the last group), as it does in a page of one tile: K's second and V's first half are one copy
+    static constexpr int  kTileBytes = (kTile / kGroupRows) * kGroupSize - (KVBITS == 4 ? kGroupPad : 0);
     static constexpr int  kParamBytes = kQuant ? kTile * 4 : 0;  // (scale, zero) as T per token
     static constexpr int  kStageBytes = 2 * kTileBytes + 2 * kParamBytes;
     // offsets inside a stage
@@ -271,32 +272,25 @@ struct KernelParams {
     int            early;  // 1: the producer warp streams KV tiles before griddepcontrol.wait, 2: the consumers look up before it, too (see the kernel's head)
 };
 
-// slot (0..15 inside a warp's 16-key MMA) -> token index inside the 64-token tile; slot c + 8 lies kNextRow tokens behind slot c
-template<int KVBITS>
-constexpr int kNextRow = KVBITS == 4 ? 8 : 1;
-template<int KVBITS>
+// slot (0..15 inside a warp's 16-key MMA) -> token index inside the 64-token tile; slot c + 8 holds the token behind that of slot c
 B200_DEVICE int slot_token(int c, int warp)
 {
-    if constexpr (KVBITS == 4) {
-        // rows of 64 bytes without padding: neighbouring rows of a fragment of K, and two of the four rows of V that a load reads, differ in parity
-        return 16 * warp + (c ^ ((c >> 1) & 1));
-    }
     // group table G = [0,2,1,3,2,0,3,1] packed 2 bits each
     const int grp = (0x72D8 >> (2 * (c & 7))) & 3;
     const int i   = (c >> 3) + 2 * ((c & 7) >> 2);
     return 16 * grp + 4 * warp + i;
 }
 // the consumer warp whose 16 keys hold a token
-template<int KVBITS>
 B200_DEVICE int token_warp(int tok)
 {
-    return KVBITS == 4 ? tok >> 4 : (tok >> 2) & 3;
+    return (tok >> 2) & 3;
 }
 
 template<int KVBITS>
 B200_DEVICE int token_smem_offset(int tok)
 {
-    return (tok >> 4) * TileCfg<KVBITS>::kGroupSize + (tok & 15) * TileCfg<KVBITS>::kRowBytes;
+    using Cfg = TileCfg<KVBITS>;
+    return tok / Cfg::kGroupRows * Cfg::kGroupSize + tok % Cfg::kGroupRows * Cfg::kRowBytes;
 }
 
 // first dim of the 4 consecutive dims lane-class t contracts in k-step j of S = K.Q^T
@@ -401,7 +395,7 @@ B200_DEVICE int merge_idx(int hd, int d)
 template<class T, int KVBITS>
 struct ConsumerCtx {
     int      warp, g, t;
-    // what belongs to slots c + 8 lies a constant away (kNextRow)
+    // what belongs to slots c + 8 lies a token behind
     int      tokA, tokV0, tokV1;     // keys of row g; of k-slots 2t, 2t + 1
     uint32_t offA, offV0, offV1;     // their rows, this lane's bytes of them included
 };
@@ -411,7 +405,7 @@ struct ConsumerCtx {
 // token's (scale, zero) are applied to the products in fp32:
 //   s_t = scale_t * 2^24 * (code_t . q) + zero_t * sum(q);    P_t = exp2(..),   P'_t = T(P_t * scale_t * kappa)
 //   kappa * O_d = 2^24 * sum_t P'_t (code_td - mid) + sum_t P'_t * (zero_t / scale_t + mid)
-// mid is the middle of the codes: the codes enter as they are, and every eight or nine tiles (kRecentre) mid * sum P' is taken off the accumulators.  Left
+// mid is the middle of the codes: the codes enter as they are, and every kRecentre tiles mid * sum P' is taken off the accumulators.  Left
 // in, it makes them a hundred times larger than the output that remains when the zero part is added, and the tensor cores cut a product's
 // bits off at the accumulator's last one (64 sequences of 8192 int8 keys: error against 64 bits 5.3e-4 with T-rounded values, 9.9e-4
 // without this, 4.5e-4 with it).
@@ -437,22 +431,22 @@ B200_DEVICE float2 half2_to_float2(uint32_t x)
     return __half22float2(reinterpret_cast<const half2&>(x));
 }
 
-template<int KVBITS>
-constexpr int kRecentre = KVBITS == 4 ? 9 : 8;  // a multiple of kTilesAtOnce
+constexpr int kRecentre = 8;  // a multiple of kTilesAtOnce
 
-// Tiles that a consumer warp takes under one maximum: their scores, then their values, are one stretch of code each, so that two chains of
-// products run beside one another, and the maxima over lanes, the vote and the loop are paid once.
-// int4 pages, 32 / 8 heads, whole operator (us, four sets of pages in turn), with two / three / four at once: 128 x 4096 f16 138.0 / 134.0 / 150 (whose
-// registers spill), bf16 161.4 / 159.9, 64 x 2048 47.4 / 47.1 / 51.5, 16 x 100 - 300 15.3 / 15.4 / 15.8; with one 128 x 4096 took 155.  int8 reads its pages at
-// 6.2 TB/s with one and gains nothing (55 us, 62 with two: only three stages fit).  T pages keep the order of sums they had.
+// Tiles that a consumer warp takes at once: their scores, then their values, are one stretch of code each, so that two chains of products run beside one
+// another, and the vote and the loop are paid once; maxima over lanes are taken only where a score lies above them.  A tile is weighed against the maximum
+// of the tiles up to it, not of those taken with it, and the sums run in the order of the tiles, so that outputs do not depend on this number.
+// int4 pages, 32 / 8 heads, whole operator (us, four sets of pages in turn), with one / two / four at once: 128 x 4096 f16 157 / 144 / 174 (four spill), bf16
+// 182 / 164 / 188, 64 x 2048 51.8 / 49.2 / 61, 16 x 100 - 300 15.3 / 15.4 / 16.0 (before tiles took fewer copies: 128 x 4096 175 and 197 in bf16, 64 x 2048 55.3,
+// 16 x 100 - 300 16.0).  int8 reads its pages at 6.2 TB/s with one and gains nothing (55 us, 62 with two: only three stages fit).
 template<int KVBITS>
-constexpr int kTilesAtOnce = KVBITS == 4 ? 3 : 1;
+constexpr int kTilesAtOnce = KVBITS == 4 ? 2 : 1;
 
 // kCodesInMma: sums that go with the accumulators of a run of tiles (heads 2t, 2t + 1)
 struct CodeSums {
     float q[2];  // q's dims
     float a[2];  // this lane's part of sum P' (zero / scale + mid)
-    float w[4];  // accumulator of P' against ones (the same for all rows g): sum P' since mid was last taken off the accumulators
+    float w[2];  // this lane's part of sum P' since mid was last taken off the accumulators
 };
 
 template<int KVBITS>
@@ -460,30 +454,18 @@ B200_DEVICE void recentre(float (&O)[8][4], CodeSums& sums)
 {
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
+        float w = sums.w[i];
+        w += __shfl_xor_sync(0xffffffffu, w, 4);
+        w += __shfl_xor_sync(0xffffffffu, w, 8);
+        w += __shfl_xor_sync(0xffffffffu, w, 16);
+        sums.w[i] = 0.f;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             const float f = CodeScale<KVBITS>::mid / CodeScale<KVBITS>::unit(j);
-            O[j][i]       = fmaf(-f, sums.w[i], O[j][i]);
-            O[j][i + 2]   = fmaf(-f, sums.w[i], O[j][i + 2]);
+            O[j][i]       = fmaf(-f, w, O[j][i]);
+            O[j][i + 2]   = fmaf(-f, w, O[j][i + 2]);
         }
     }
-    sums.w[0] = sums.w[1] = sums.w[2] = sums.w[3] = 0.f;
-}
-
-// (scale, zero) of a token and of the one kNextRow behind it
-template<int KVBITS>
-B200_DEVICE uint2 params2(uint32_t addr)
-{
-    if constexpr (kNextRow<KVBITS> == 1) {
-        return lds64(addr);
-    }
-    return make_uint2(lds32(addr), lds32(addr + 4 * kNextRow<KVBITS>));
-}
-B200_DEVICE float rcp_approx(float x)
-{
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
 }
 
 // scores of this warp's 16 keys of a tile.  `st` = shared address of the stage.  S[0], S[1]: row g (tokA) heads 2t, 2t + 1;  S[2], S[3]: row g + 8 (tokB)
@@ -493,11 +475,11 @@ B200_DEVICE void score_tile(const ConsumerCtx<T, KVBITS>& cx, uint32_t st, const
     using Ops = TypeOps<T>;
     using Cfg = TileCfg<KVBITS>;
     const int t = cx.t;
-    const int tokA = cx.tokA, tokB = cx.tokA + kNextRow<KVBITS>;
-    const uint32_t rowA = st + Cfg::kOffK + cx.offA, rowB = rowA + kNextRow<KVBITS> * Cfg::kRowBytes;
+    const int tokA = cx.tokA, tokB = cx.tokA + 1;
+    const uint32_t rowA = st + Cfg::kOffK + cx.offA, rowB = rowA + Cfg::kRowBytes;
     S[0] = S[1] = S[2] = S[3] = 0.f;
     if constexpr (kCodesInMma<T, KVBITS>) {
-        const uint2  kp = params2<KVBITS>(st + Cfg::kOffKP + tokA * 4);
+        const uint2  kp = lds64(st + Cfg::kOffKP + tokA * 4);
         const float2 zA = half2_to_float2(kp.x), zB = half2_to_float2(kp.y);
         if constexpr (KVBITS == 8) {
             uint4 ka[2], kb[2];
@@ -609,8 +591,8 @@ B200_DEVICE void grow_maxima(const float (&mx)[2], float c, float (&O)[8][4], fl
         L[0] *= r0;
         L[1] *= r1;
         if constexpr (kCodesInMma<T, KVBITS>) {
-            sums.a[0] *= r0, sums.w[0] *= r0, sums.w[2] *= r0;
-            sums.a[1] *= r1, sums.w[1] *= r1, sums.w[3] *= r1;
+            sums.a[0] *= r0, sums.w[0] *= r0;
+            sums.a[1] *= r1, sums.w[1] *= r1;
         }
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
@@ -640,7 +622,7 @@ struct ValueRows {
     uint32_t row0, row1, row2, row3;  // of k-slots 2t, 2t + 1, 2t + 8, 2t + 9
     B200_DEVICE ValueRows(const ConsumerCtx<T, KVBITS>& cx, uint32_t st)
     {
-        constexpr int next = kNextRow<KVBITS> * TileCfg<KVBITS>::kRowBytes;
+        constexpr int next = TileCfg<KVBITS>::kRowBytes;
         row0 = st + TileCfg<KVBITS>::kOffV + cx.offV0, row1 = st + TileCfg<KVBITS>::kOffV + cx.offV1;
         row2 = row0 + next, row3 = row1 + next;
     }
@@ -653,7 +635,7 @@ struct ValueParams {
 template<class T, int KVBITS>
 B200_DEVICE ValueParams value_params(const ConsumerCtx<T, KVBITS>& cx, uint32_t st)
 {
-    const uint2 vp = params2<KVBITS>(st + TileCfg<KVBITS>::kOffVP + cx.tokA * 4);
+    const uint2 vp = lds64(st + TileCfg<KVBITS>::kOffVP + cx.tokA * 4);
     return {half2_to_float2(vp.x), half2_to_float2(vp.y)};
 }
 // the values' codes may go into the product as they are
@@ -673,13 +655,13 @@ B200_DEVICE void weigh_codes(const ConsumerCtx<T, KVBITS>& cx, uint32_t st, cons
     const auto [row0, row1, row2, row3] = ValueRows<T, KVBITS>(cx, st);
     const float    kA = v.A.x * CS::kappa, kB = v.B.x * CS::kappa;
     const uint32_t wA = Ops::pack2(P[0] * kA, P[1] * kA), wB = Ops::pack2(P[2] * kB, P[3] * kB);
-    const float    rA = fmaf(v.A.y, rcp_approx(v.A.x), CS::mid), rB = fmaf(v.B.y, rcp_approx(v.B.x), CS::mid);
+    const float    rA = __fdividef(v.A.y, v.A.x) + CS::mid, rB = __fdividef(v.B.y, v.B.x) + CS::mid;
     const float2   fA = half2_to_float2(wA), fB = half2_to_float2(wB);
     sums.a[0] = fmaf(fA.x, rA, fmaf(fB.x, rB, sums.a[0]));
     sums.a[1] = fmaf(fA.y, rA, fmaf(fB.y, rB, sums.a[1]));
-    const uint32_t pf[2]   = {transpose_8x8_b16(wA), transpose_8x8_b16(wB)};
-    const uint32_t ones[4] = {0x3c003c00u, 0x3c003c00u, 0x3c003c00u, 0x3c003c00u};
-    Ops::mma16816(sums.w, ones, pf);
+    sums.w[0] += fA.x + fB.x;
+    sums.w[1] += fA.y + fB.y;
+    const uint32_t pf[2] = {transpose_8x8_b16(wA), transpose_8x8_b16(wB)};
     if constexpr (KVBITS == 8) {
         const uint4 v0 = lds128(row0), v1 = lds128(row1);
         const uint4 v2 = lds128(row2), v3 = lds128(row3);
@@ -719,7 +701,7 @@ B200_DEVICE void weigh_rounded(const ConsumerCtx<T, KVBITS>& cx, uint32_t st, bo
 {
     using Ops = TypeOps<T>;
     using Cfg = TileCfg<KVBITS>;
-    const int  tokV0 = cx.tokV0, tokV1 = cx.tokV1, tokV2 = cx.tokV0 + kNextRow<KVBITS>, tokV3 = cx.tokV1 + kNextRow<KVBITS>;
+    const int  tokV0 = cx.tokV0, tokV1 = cx.tokV1, tokV2 = cx.tokV0 + 1, tokV3 = cx.tokV1 + 1;
     const auto [row0, row1, row2, row3] = ValueRows<T, KVBITS>(cx, st);
     uint32_t pf[2];
     pf[0] = transpose_8x8_b16(Ops::pack2(P[0], P[1]));  // k-slots 2t,2t+1 ; head g
@@ -847,7 +829,7 @@ B200_DEVICE void weigh_tile(const ConsumerCtx<T, KVBITS>& cx, uint32_t st, bool 
         if (residue && t0 + cx.tokA >= k_len) {
             v.A = make_float2(CodeScale<KVBITS>::kMin, 0.f);
         }
-        if (residue && t0 + cx.tokA + kNextRow<KVBITS> >= k_len) {
+        if (residue && t0 + cx.tokA + 1 >= k_len) {
             v.B = make_float2(CodeScale<KVBITS>::kMin, 0.f);
         }
         if (__all_sync(0xffffffffu, fit<KVBITS>(v))) {
@@ -878,7 +860,7 @@ B200_DEVICE void process_tile(const ConsumerCtx<T, KVBITS>& cx, uint32_t st, boo
     if (residue && (t0 + cx.tokA >= k_len)) {
         S[0] = S[1] = -INFINITY;
     }
-    if (residue && (t0 + cx.tokA + kNextRow<KVBITS> >= k_len)) {
+    if (residue && (t0 + cx.tokA + 1 >= k_len)) {
         S[2] = S[3] = -INFINITY;
     }
     float mx[2] = {fmaxf(S[0], S[2]), fmaxf(S[1], S[3])};
@@ -890,46 +872,55 @@ B200_DEVICE void process_tile(const ConsumerCtx<T, KVBITS>& cx, uint32_t st, boo
     weigh_tile<T, KVBITS>(cx, st, residue, k_len, t0, P, O, sums);
 }
 
-// NT tiles, all keys of which are seen, with one maximum for all of them: `st` = shared addresses of their stages
+// NT tiles, all keys of which are seen, as process_tile would take them one after the other: `st` = shared addresses of their stages
 template<class T, int KVBITS, int NT>
 B200_DEVICE void process_tiles(const ConsumerCtx<T, KVBITS>& cx, const uint32_t (&st)[NT], float c, const uint32_t (&qf)[8][2], float (&O)[8][4],
                                float (&M)[2], float (&L)[2], CodeSums& sums)
 {
-    float S[NT][4], mx[2] = {-INFINITY, -INFINITY};
+    float S[NT][4], mx[NT][2];
+    bool  grow = false;
 #pragma unroll
     for (int i = 0; i < NT; ++i) {
         score_tile<T, KVBITS>(cx, st[i], qf, sums, S[i]);
-        mx[0] = fmaxf(mx[0], fmaxf(S[i][0], S[i][2]));
-        mx[1] = fmaxf(mx[1], fmaxf(S[i][1], S[i][3]));
+        mx[i][0] = fmaxf(S[i][0], S[i][2]), mx[i][1] = fmaxf(S[i][1], S[i][3]);
+        grow = grow || mx[i][0] > M[0] || mx[i][1] > M[1];
     }
-    warp_maxima(mx);
-    grow_maxima<T, KVBITS>(mx, c, O, M, L, sums);
-    const float mc0 = M[0] == -INFINITY ? 0.f : M[0] * c, mc1 = M[1] == -INFINITY ? 0.f : M[1] * c;
+    grow = __any_sync(0xffffffffu, grow);
+    if (grow) {
 #pragma unroll
-    for (int i = 0; i < NT; ++i) {
-        float P[4];
+        for (int i = 0; i < NT; ++i) warp_maxima(mx[i]);
+    }
+    auto weights_of = [&](int i, float (&P)[4]) {
+        if (grow) {
+            grow_maxima<T, KVBITS>(mx[i], c, O, M, L, sums);
+        }
+        const float mc0 = M[0] == -INFINITY ? 0.f : M[0] * c, mc1 = M[1] == -INFINITY ? 0.f : M[1] * c;
         weights(S[i], c, mc0, mc1, P, L);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) S[i][k] = P[k];
-    }
+    };
     if constexpr (kCodesInMma<T, KVBITS>) {
         uint2 raw[NT];
         bool  ok = true;
 #pragma unroll
         for (int i = 0; i < NT; ++i) {
-            raw[i] = params2<KVBITS>(st[i] + TileCfg<KVBITS>::kOffVP + cx.tokA * 4);
+            raw[i] = lds64(st[i] + TileCfg<KVBITS>::kOffVP + cx.tokA * 4);
             ok     = ok && fit<KVBITS>(ValueParams{half2_to_float2(raw[i].x), half2_to_float2(raw[i].y)});
         }
         if (__all_sync(0xffffffffu, ok)) {
 #pragma unroll
             for (int i = 0; i < NT; ++i) {
-                weigh_codes<T, KVBITS>(cx, st[i], ValueParams{half2_to_float2(raw[i].x), half2_to_float2(raw[i].y)}, S[i], O, sums);
+                float P[4];
+                weights_of(i, P);
+                weigh_codes<T, KVBITS>(cx, st[i], ValueParams{half2_to_float2(raw[i].x), half2_to_float2(raw[i].y)}, P, O, sums);
             }
             return;
         }
     }
 #pragma unroll
-    for (int i = 0; i < NT; ++i) weigh_tile<T, KVBITS>(cx, st[i], false, 0, 0, S[i], O, sums);
+    for (int i = 0; i < NT; ++i) {
+        float P[4];
+        weights_of(i, P);
+        weigh_tile<T, KVBITS>(cx, st[i], false, 0, 0, P, O, sums);
+    }
 }
 
 B200_DEVICE void sts32(uint32_t addr, uint32_t v)
@@ -1217,11 +1208,12 @@ __global__ void __launch_bounds__(kThreads, min_ctas_per_sm<KVBITS>()) decode_at
         for (long long base = lo; base < hi; base += 32) {
             const TileDesc nxt = fetch(base + 32);
             const int      cnt = (int)min((long long)32, hi - base);
-            if constexpr (Cfg::kGroupPad == 0) {
-                // The lane that holds a tile's descriptor issues its copies: two of them where a page is one tile long, four otherwise.  A bulk copy
-                // takes its operands from uniform registers, so that lanes which issue together are served one after the other: ten copies per
+            if constexpr (KVBITS == 4) {
+                // The lane that holds a tile's descriptor issues its copies: four of them where a page is one tile long, up to six otherwise.  A bulk
+                // copy takes its operands from uniform registers, so that lanes which issue together are served one after the other: ten copies per
                 // tile cost this warp some 450 issue slots and up to 1290 cycles (consumers that only wait and release: 110 us for 128 x 4096 int4
-                // keys, whose bytes take 88).  With this and the rows without padding it needs: 166 -> 140 us.
+                // keys, whose bytes take 88; the whole 166, with these copies 144).  Two copies into rows without any padding, whose products then
+                // take rows in another order and put the scores back: 148.
                 const char*    data   = cur.blk + (size_t)cur.h * 2 * head_data_size + (size_t)cur.bt * Cfg::kRowBytes;
                 const char*    par    = cur.blk + (size_t)Hkv * 2 * head_data_size + (size_t)cur.h * 2 * head_param_sz + (size_t)cur.bt * 4;
                 const int      rows   = cur.rows & 127;
@@ -1237,13 +1229,21 @@ __global__ void __launch_bounds__(kThreads, min_ctas_per_sm<KVBITS>()) decode_at
                         mbar_wait(empty0 + 8 * s, ph ^ 1);
                         const int n = rows * Cfg::kRowBytes, np = ((rows + 3) & ~3) * 4;
                         mbar_expect_tx(bar, 2 * (n + np));
+                        constexpr int half = kTile / 2 * Cfg::kRowBytes;
                         if (rows == kTile && p.block_len == kTile) {
-                            bulk_g2s_hint(st + Cfg::kOffK, data, 2 * Cfg::kTileBytes, bar, policy);
+                            bulk_g2s_hint(st + Cfg::kOffK, data, half, bar, policy);
+                            bulk_g2s_hint(st + Cfg::kOffK + Cfg::kGroupSize, data + half, 2 * half, bar, policy);
+                            bulk_g2s_hint(st + Cfg::kOffV + Cfg::kGroupSize, data + 3 * half, half, bar, policy);
                             bulk_g2s_hint(st + Cfg::kOffKP, par, 2 * Cfg::kParamBytes, bar, policy);
                         }
                         else {
-                            bulk_g2s_hint(st + Cfg::kOffK, data, n, bar, policy);
-                            bulk_g2s_hint(st + Cfg::kOffV, data + head_data_size, n, bar, policy);
+                            const int n0 = min(n, half);
+                            bulk_g2s_hint(st + Cfg::kOffK, data, n0, bar, policy);
+                            bulk_g2s_hint(st + Cfg::kOffV, data + head_data_size, n0, bar, policy);
+                            if (n > n0) {
+                                bulk_g2s_hint(st + Cfg::kOffK + Cfg::kGroupSize, data + half, n - n0, bar, policy);
+                                bulk_g2s_hint(st + Cfg::kOffV + Cfg::kGroupSize, data + head_data_size + half, n - n0, bar, policy);
+                            }
                             bulk_g2s_hint(st + Cfg::kOffKP, par, np, bar, policy);
                             bulk_g2s_hint(st + Cfg::kOffVP, par + head_param_sz, np, bar, policy);
                         }
@@ -1276,10 +1276,10 @@ __global__ void __launch_bounds__(kThreads, min_ctas_per_sm<KVBITS>()) decode_at
                 const uint32_t st = stage0 + s * (uint32_t)Cfg::kStageBytes;
                 const char*    hb = reinterpret_cast<const char*>(blk);
                 if (my_data) {
-                    const int r = min(kGroupRows, rows - my_gq * kGroupRows);
+                    const int r = min(Cfg::kGroupRows, rows - my_gq * Cfg::kGroupRows);
                     if (r > 0) {
                         const char* src = hb + (size_t)(h * 2 + (my_v ? 1 : 0)) * head_data_size
-                                          + (size_t)(bt + my_gq * kGroupRows) * Cfg::kRowBytes;
+                                          + (size_t)(bt + my_gq * Cfg::kGroupRows) * Cfg::kRowBytes;
                         bulk_g2s_hint(st + (my_v ? Cfg::kOffV : Cfg::kOffK) + my_gq * Cfg::kGroupSize, src,
                                       r * Cfg::kRowBytes, bar, policy);
                     }
@@ -1306,8 +1306,8 @@ __global__ void __launch_bounds__(kThreads, min_ctas_per_sm<KVBITS>()) decode_at
     cx.g    = lane >> 2;
     cx.t    = lane & 3;
     const int g = cx.g, t = cx.t;
-    cx.tokA  = slot_token<KVBITS>(g, warp);
-    cx.tokV0 = slot_token<KVBITS>(2 * t, warp), cx.tokV1 = slot_token<KVBITS>(2 * t + 1, warp);
+    cx.tokA  = slot_token(g, warp);
+    cx.tokV0 = slot_token(2 * t, warp), cx.tokV1 = slot_token(2 * t + 1, warp);
     cx.offA  = token_smem_offset<KVBITS>(cx.tokA) + 16 * t;
     cx.offV0 = token_smem_offset<KVBITS>(cx.tokV0) + (KVBITS == 4 ? 8 : 16) * g;
     cx.offV1 = token_smem_offset<KVBITS>(cx.tokV1) + (KVBITS == 4 ? 8 : 16) * g;
@@ -1377,7 +1377,7 @@ __global__ void __launch_bounds__(kThreads, min_ctas_per_sm<KVBITS>()) decode_at
             M[0] = M[1] = -INFINITY;
             L[0] = L[1] = 0.f;
             if constexpr (kCodesInMma<T, KVBITS>) {
-                sums.a[0] = sums.a[1] = sums.w[0] = sums.w[1] = sums.w[2] = sums.w[3] = 0.f;
+                sums.a[0] = sums.a[1] = sums.w[0] = sums.w[1] = 0.f;
                 float q = 0.f;  // head g: this lane's 32 dims, then all 128
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
@@ -1397,7 +1397,7 @@ __global__ void __launch_bounds__(kThreads, min_ctas_per_sm<KVBITS>()) decode_at
         // before a tile, not behind it: the peeled form takes the same steps
         auto recentre_at = [&](int tt) {
             if constexpr (kCodesInMma<T, KVBITS>) {
-                if (tt > 0 && tt % kRecentre<KVBITS> == 0) {
+                if (tt > 0 && tt % kRecentre == 0) {
                     recentre<KVBITS>(O, sums);
                 }
             }
@@ -1405,7 +1405,7 @@ __global__ void __launch_bounds__(kThreads, min_ctas_per_sm<KVBITS>()) decode_at
         int tt = 0;
         if constexpr (kTilesAtOnce<KVBITS> > 1) {
             constexpr int NT   = kTilesAtOnce<KVBITS>;
-            static_assert(kRecentre<KVBITS> % NT == 0, "the sums are centred between two turns");
+            static_assert(kRecentre % NT == 0, "the sums are centred between two turns");
             const int     many = min(nloop, it.tiles - 1 - first_tile);  // a sequence's last tile may end early
             for (; tt + NT <= many; tt += NT) {
                 recentre_at(tt);
@@ -1450,11 +1450,11 @@ __global__ void __launch_bounds__(kThreads, min_ctas_per_sm<KVBITS>()) decode_at
             const int t0 = (it.tiles - 1) * kTile;
             recentre_at(nloop);
             mbar_wait(full0 + 8 * s, ph);
-            // The new token's slot belongs to exactly one consumer warp (slot_token: token & 15 = 4 * warp + i): that warp runs
+            // The new token's slot belongs to exactly one consumer warp (token_warp): that warp runs
             // the prologue for this (sequence, kv-head) -- bias, RoPE(k), quantise, store into the page for later steps -- and
             // overwrites the row the bulk copy brought in (stale bytes) in ITS OWN view of the tile; no other warp reads it.
             const int pos = k_len - 1 - t0;
-            if (token_warp<KVBITS>(pos) == warp) {
+            if (token_warp(pos) == warp) {
                 new_token_kv<T, KVBITS>(p, it.b, it.h, k_len - 1, pos, lane, stage0 + s * (uint32_t)Cfg::kStageBytes);
                 __syncwarp();
             }

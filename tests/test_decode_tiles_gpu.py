@@ -1,6 +1,6 @@
-"""Decode attention over int4 pages, whose consumer warps take three tiles of 64 keys at a time: runs of tiles that end on either side of three and of a sequence's
-last tile, pages of one and of two tiles (copied in two and in four parts), values whose scales let codes through as they are in all, some or none of
-three tiles.  Many sequences share one history, so that a CTA has dozens of tiles in a row; against 64 bits."""
+"""Decode attention over int4 pages, whose consumer warps take two tiles of 64 keys at a time: runs of tiles that end on either side of two and of a sequence's
+last tile, pages of one and of two tiles (copied in four and in six parts), values whose scales let codes through as they are in all, some or none of
+the tiles, scores that grow from tile to tile.  Many sequences share one history, so that a CTA has dozens of tiles in a row; against 64 bits."""
 import ctypes as C
 
 import numpy as np
@@ -53,8 +53,8 @@ def test_tiles_at_once(hist, block_len, G, dtype, odd, lib, monkeypatch):
     case = PagedCase(batch_hist=[hist], num_heads=G, num_kv_heads=1, kv_bits=4, block_len=block_len, dtype=dtype, seed=G, rope=OA.RopeParam(type=OA.ROPE_NULL))
     rng = np.random.default_rng(hist)
     tok = np.arange(hist)[:, None, None]
-    # constant vectors (scale 0) do not go through as codes: one warp's keys of every third tile; every third tile; all
-    flat = {"none": tok < 0, "warps": (tok // 64 % 3 == 1) & (tok // 16 % 4 == 2), "tiles": tok // 64 % 3 == 1, "all": tok >= 0}[odd]
+    # constant vectors (scale 0) do not go through as codes: one warp's keys (four groups of four, 16 apart) of every third tile; every third tile; all
+    flat = {"none": tok < 0, "warps": (tok // 64 % 3 == 1) & (tok // 4 % 4 == 2), "tiles": tok // 64 % 3 == 1, "all": tok >= 0}[odd]
     k = rn(rng.standard_normal((hist, 1, 128)).astype(np.float32), dtype)
     v = rn(np.where(flat, 0.25 + tok % 7, rng.standard_normal((hist, 1, 128))).astype(np.float32), dtype)
     OA.process_kv(case.cache, case.block_tables[0], case.layer, 0, k, v, case.rope, None, None)
@@ -79,3 +79,25 @@ def test_tiles_at_once(hist, block_len, G, dtype, odd, lib, monkeypatch):
         bar = (p * (2 + 2 * score)) @ np.abs(Vb) * u + u * np.abs(ref) + 2.0 ** -18 * np.abs(Vb).max() + 2.0 ** -24
         err = np.abs(got[b] - ref)
         assert (err <= bar).all(), (b, float((err / bar).max()))
+
+
+@pytest.mark.parametrize("tile", [1, 2])
+@pytest.mark.parametrize("at", [0, 3])
+def test_a_tile_is_weighed_against_the_maxima_up_to_it(tile, at, lib):
+    """Narrow values far from zero in the first tiles, zeros (in every other dimension) behind them, and in the first tile behind them a key of each warp whose
+    score is 22 octaves above all others.  Weighed against the maximum of its own time a tile's weights are twice the least scale, rounded to 11 bits;
+    against the loud keys', which come later, they would be subnormal numbers of 8.5 steps."""
+    hist, G = 4095, 4
+    case = PagedCase(batch_hist=[hist], num_heads=G, num_kv_heads=1, kv_bits=4, seed=1, rope=OA.RopeParam(type=OA.ROPE_NULL))
+    k, v = np.zeros((hist, 1, 128), np.float32), np.zeros((hist, 1, 128), np.float32)
+    v[:64 * tile] = 1.5
+    v[:, :, ::2] += 2.0 ** -9                                               # scale 2^-9 / 15; from 2^-14 on codes go through as they are
+    k[64 * tile + at + np.array([0, 20, 40, 60]), 0, 0] = 15.0
+    OA.process_kv(case.cache, case.block_tables[0], case.layer, 0, k, v, case.rope, None, None)
+    qkv = np.zeros((BATCH, (G + 2) * 128), np.float32)
+    q = float(rn(np.float32(22 * np.log(2.0) * np.sqrt(128.0) / 15.0), F16))
+    qkv[:, :G * 128:128] = q
+    got, w = _run(case, lib, qkv, G)[:, :, 1::2], np.exp(-15.0 * q / np.sqrt(128.0))
+    ref = 64 * tile * 1.5 * w / (4 + (hist + 1 - 4) * w)
+    # the weights' rounding (2^-11), float sums in which parts some 20 times as large cancel, and the result's half step
+    assert (np.abs(got - ref) <= 2.0 ** -10 * ref + 2.0 ** -25).all(), float(np.abs(got / ref - 1).max())
