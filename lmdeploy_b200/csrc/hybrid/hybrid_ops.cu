@@ -470,7 +470,8 @@ __global__ void gated_rms_kernel(const float* __restrict__ o, const float* __res
 // Router: logits = router x + bias (float; bias nullptr: none); scores = softmax over all experts (score_fn 0), the sigmoid of every
 // logit on its own (score_fn 1) or softmax over the chosen logits only (score_fn 2); the `top` largest (ties: the lower index), their
 // scores as weights.  x is float or T.
-template <typename TI>
+// DEPTH weights of a warp's lane are in flight at once; 0: sixteen, in the compiler's way (route_depth).
+template <typename TI, int DEPTH>
 __global__ void route_kernel(const TI* __restrict__ x, const float* __restrict__ router, const float* __restrict__ bias, int width, int experts,
                              int top, int score_fn, int* __restrict__ ids, float* __restrict__ wts)
 {
@@ -480,29 +481,42 @@ __global__ void route_kernel(const TI* __restrict__ x, const float* __restrict__
     float* chosen = z + experts;                              // [top]
     b200::pdl_launch_dependents();                            // the experts' blocks set themselves up meanwhile, and wait for this kernel's end
     const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    // A warp's 2048 weights are all in flight at once, the first of them beside the row of x: what bounds this kernel is the number of memory
-    // latencies in a row (with sixteen reads in flight behind x: 11.3 us for 32 rows of 2048 x 8 experts, 8.4 so; the same sums in the same order).
-    constexpr int DEEP = 64;
-    float v[DEEP];
-    auto ask = [&](int e, int i0) {
-        const float* row = router + (size_t)e * width + i0 + lane;
-#pragma unroll
-        for (int j = 0; j < DEEP; ++j) v[j] = i0 + lane + 32 * j < width ? row[32 * j] : 0.f;
-    };
-    if (warp < experts) ask(warp, 0);
-#pragma unroll 8
-    for (int i = threadIdx.x; i < width; i += blockDim.x) xs[i] = to_f(x[(size_t)t * width + i]);
-    __syncthreads();
-    for (int e = warp; e < experts; e += nw) {
-        float part = 0.f;
-        for (int i0 = 0; i0 < width; i0 += 32 * DEEP) {
-            if (e != warp || i0 > 0) ask(e, i0);
-#pragma unroll
-            for (int j = 0; j < DEEP; ++j)
-                if (i0 + lane + 32 * j < width) part = fmaf(v[j], xs[i0 + lane + 32 * j], part);
-        }
+    auto result = [&](int e, float part) {
         part = warp_sum(part);
         if (lane == 0) z[e] = part + (bias ? bias[e] : 0.f);
+    };
+    if constexpr (DEPTH == 0) {
+#pragma unroll 4
+        for (int i = threadIdx.x; i < width; i += blockDim.x) xs[i] = to_f(x[(size_t)t * width + i]);
+        __syncthreads();
+        for (int e = warp; e < experts; e += nw) {
+            const float* row = router + (size_t)e * width;
+            float part = 0.f;
+#pragma unroll 16
+            for (int i = lane; i < width; i += 32) part = fmaf(row[i], xs[i], part);
+            result(e, part);
+        }
+    } else {
+        float v[DEPTH];                                       // the first expert's beside the row of x
+        auto ask = [&](int e, int i0) {
+            const float* row = router + (size_t)e * width + i0 + lane;
+#pragma unroll
+            for (int j = 0; j < DEPTH; ++j) v[j] = i0 + lane + 32 * j < width ? row[32 * j] : 0.f;
+        };
+        if (warp < experts) ask(warp, 0);
+#pragma unroll 8
+        for (int i = threadIdx.x; i < width; i += blockDim.x) xs[i] = to_f(x[(size_t)t * width + i]);
+        __syncthreads();
+        for (int e = warp; e < experts; e += nw) {
+            float part = 0.f;
+            for (int i0 = 0; i0 < width; i0 += 32 * DEPTH) {
+                if (e != warp || i0 > 0) ask(e, i0);
+#pragma unroll
+                for (int j = 0; j < DEPTH; ++j)
+                    if (i0 + lane + 32 * j < width) part = fmaf(v[j], xs[i0 + lane + 32 * j], part);
+            }
+            result(e, part);
+        }
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -1198,13 +1212,27 @@ B200H_API int b200h_gated_rms(const void* o, const void* w, const void* gate, in
     return launched("gated_rms");
 }
 
+// For few rows the number of memory latencies in a row bounds the router: all 2048 weights of a warp in flight (86 registers, two blocks per SM).  For many
+// rows it is the blocks in flight, and for narrow rows the 64 steps that are taken whatever the width: sixteen reads in flight (40 registers, six blocks).
+// Same sums in the same order.  us, sixteen / 64, 8 experts: 2048 wide, 32 rows 14.6 / 8.5, 1024 rows 27 / 19, 4096 rows 73 / 85; 4096 wide, 2048 rows 76 / 71,
+// 4096 rows 135 / 150; 768 wide, 512 rows 9 / 9, 1024 rows 13 / 15; 256 wide, 4096 rows 15 / 38.  64 experts: 2048 wide, 32 rows 86 / 19, 8192 rows 856 / 548; 1408
+// wide, 8192 rows 628 / 500; 1024 wide, 8192 rows 452 / 459; 512 wide, 256 rows 29 / 21, 512 rows 29 / 35, 4096 rows 83 / 214; 64 wide, 1 row 12 / 15, 4096 rows 48 / 209.
+// 16 experts: 2048 wide, 8192 rows 233 / 206; 1408 wide, 4096 rows 53 / 69.
+static int route_depth(int n, int width, int experts)
+{
+    const bool few  = width >= 256 && 4 * (int64_t)n <= 3 * (int64_t)width;
+    const bool many_experts = (int64_t)experts * width >= 32768 && (width >= 1408 ? experts >= 16 : width >= 1024 && experts >= 64);
+    return few || many_experts ? 64 : 0;
+}
+
 template <typename TI>
 static void launch_route(const void* x, const void* router, const void* bias, int n, int width, int experts, int top, int score_fn, void* ids,
                          void* wts, size_t smem, cudaStream_t st)
 {
-    if (smem > 48 * 1024) cudaFuncSetAttribute(route_kernel<TI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    route_kernel<TI><<<n, 256, smem, st>>>((const TI*)x, (const float*)router, (const float*)bias, width, experts, top, score_fn, (int*)ids,
-                                            (float*)wts);
+    auto* kernel = route_depth(n, width, experts) ? &route_kernel<TI, 64> : &route_kernel<TI, 0>;
+    if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    kernel<<<n, 256, smem, st>>>((const TI*)x, (const float*)router, (const float*)bias, width, experts, top, score_fn, (int*)ids,
+                                 (float*)wts);
 }
 
 B200H_API int b200h_route_scored(const void* x, int x_dtype, const void* router, const void* bias, int n, int width, int experts, int top,
