@@ -883,31 +883,42 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const Params p)
         const int    tid  = threadIdx.x - 64;  // 0 .. 32 * kDqWarps - 1
         const float* base = p.partials + (size_t)blockIdx.x * p.splits * p.MT * ROWS + (size_t)t_lo * ROWS;
         if (p.epilogue != 2) {
-            for (int idx = tid; idx < (t_hi - t_lo) * (ROWS / 4); idx += kDqWarps * 32) {
-                const int     tl = idx / (ROWS / 4), nq = idx - tl * (ROWS / 4);
-                float4        acc = make_float4(0.f, 0.f, 0.f, 0.f);
-                const float4* src = reinterpret_cast<const float4*>(base + tl * ROWS) + nq;
-                // Four rows of a token per item, all of a split's partials in flight (up to eight), summed in split order: deterministic.  One round of
-                // loads instead of two (64 tokens, eight splits; this phase 3.4 k -> 2.7 k cycles): fp8 8192 x 7168 gated, 64 tokens, 26.9 -> 25.8 us, u4
-                // 14336 x 4096 20.7 -> 20.1.  Row-major partials [row][token], written and read 16 - 32 bytes a lane at a row's stride, take 8.4 k
-                // cycles: a line per lane.
-                for (int r0 = 0; r0 < p.splits; r0 += 8) {
-                    float4 v[8];
+            // Four rows of a token per item, all of a split's partials in flight (up to eight), summed in split order: deterministic.  One round of
+            // loads instead of two (64 tokens, eight splits; this phase 3.4 k -> 2.7 k cycles): fp8 8192 x 7168 gated, 64 tokens, 26.9 -> 25.8 us, u4
+            // 14336 x 4096 20.7 -> 20.1.  Row-major partials [row][token], written and read 16 - 32 bytes a lane at a row's stride, take 8.4 k
+            // cycles: a line per lane.
+            auto reduce = [&](auto load4) {
+                for (int idx = tid; idx < (t_hi - t_lo) * (ROWS / 4); idx += kDqWarps * 32) {
+                    const int    tl = idx / (ROWS / 4), nq = idx - tl * (ROWS / 4);
+                    float4       acc = make_float4(0.f, 0.f, 0.f, 0.f);
+                    const float* src = base + tl * ROWS + 4 * nq;
+                    for (int r0 = 0; r0 < p.splits; r0 += 8) {
+                        float4 v[8];
 #pragma unroll
-                    for (int r = 0; r < 8; ++r) {
-                        if (r0 + r < p.splits) {
-                            v[r] = __ldcg(src + (size_t)(r0 + r) * (p.MT * ROWS / 4));
+                        for (int r = 0; r < 8; ++r) {
+                            if (r0 + r < p.splits) {
+                                v[r] = load4(src + (size_t)(r0 + r) * (p.MT * ROWS));
+                            }
+                        }
+#pragma unroll
+                        for (int r = 0; r < 8; ++r) {
+                            if (r0 + r < p.splits) {
+                                acc.x += v[r].x, acc.y += v[r].y, acc.z += v[r].z, acc.w += v[r].w;
+                            }
                         }
                     }
-#pragma unroll
-                    for (int r = 0; r < 8; ++r) {
-                        if (r0 + r < p.splits) {
-                            acc.x += v[r].x, acc.y += v[r].y, acc.z += v[r].z, acc.w += v[r].w;
-                        }
-                    }
+                    finalize_pair<T>(p, t_lo + tl, nt0 * kBN + 4 * nq, acc.x, acc.y);
+                    finalize_pair<T>(p, t_lo + tl, nt0 * kBN + 4 * nq + 2, acc.z, acc.w);
                 }
-                finalize_pair<T>(p, t_lo + tl, nt0 * kBN + 4 * nq, acc.x, acc.y);
-                finalize_pair<T>(p, t_lo + tl, nt0 * kBN + 4 * nq + 2, acc.z, acc.w);
+            };
+            if (((uintptr_t)p.partials & 15) == 0) {
+                reduce([](const float* q) { return __ldcg(reinterpret_cast<const float4*>(q)); });
+            }
+            else {  // packed activations come from elsewhere: nothing asks more of the workspace than multiples of eight bytes
+                reduce([](const float* q) {
+                    const float2 a = __ldcg(reinterpret_cast<const float2*>(q)), b = __ldcg(reinterpret_cast<const float2*>(q) + 1);
+                    return make_float4(a.x, a.y, b.x, b.y);
+                });
             }
         }
         else {
