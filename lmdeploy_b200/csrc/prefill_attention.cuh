@@ -33,7 +33,7 @@
 //   the same, queries fetched by the loaders a piece ahead (3 us of each piece before), outputs read at once        166 / 224
 //   128-byte swizzle: eight lanes copy a line to a line                                                             144 / 189  (148 / 197 without the turns)
 //   two floats per multiplication, fewer instructions per copy, columns of a rescale read ahead                     140 / 186
-//   the prologue's heads by kind, a merge whose blocks are resident at once                                        131 / 182
+//   the prologue's heads by kind, a merge with 16 dims a thread                                                    131 / 182
 // All of them agree bit for bit.  A step takes some 4 k cycles where the tensor pipe needs 2.0 k and the exponentials 2.0 k: the chain of
 // a tile (scores, maximum, rescaled accumulator, weights: 64 % of all issue slots) bounds it.  Without any rescale 170 us, without any exponential
 // 171 (one prompt of 2048 behind 4096, 189 with both).
@@ -161,33 +161,12 @@ struct PrefillRows: PrefillRowMap<KVBITS> {
     using Map::half_of;
     using Map::key_of;
     using Map::unit_of;
-    using Lines = PrefillLineMap;
     static constexpr int kRow = Map::kRow, kInstr = Map::kInstr, kIter = Map::kIter;
-    uint32_t par[kIter];  // quantised pages: (scale, zero) of the thread's rows
+    uint32_t par[kIter];  // (scale, zero) of the thread's rows
 
-    // asynchronous 16-byte copies of the tile's rows: T pages straight into the operand tile `dst`, quantised ones into the staging
-    // tile `dst`, where instruction i of the tile has 512 bytes of its own
+    // asynchronous 16-byte copies of the tile's rows into the staging tile `dst`, where instruction i of the tile has 512 bytes of its own
     B200_DEVICE void fetch(const PrefillParams& p, const PrefillKeyTile& x, int is_v, uint32_t dst, int w, int lane)
     {
-        if constexpr (KVBITS == 16) {
-            const uint32_t to   = dst + Lines::place(w, lane);
-            const int64_t  from = is_v * p.block_len * kRow + Lines::unit0(lane) * 16;
-            const int      last = x.last - x.j * kPfKeys;
-#pragma unroll
-            for (int it = 0; it < Lines::kIter; ++it) {
-                const int row = Lines::row_of(w, lane, it);
-                if (it + 1 == Lines::kIter && !Lines::inside(w, it)) {
-                    break;
-                }
-                const int      n   = row <= last ? 16 : 0;
-                const char*    src = (Lines::row_of(w, 0, it) < 64 ? x.data0 : x.data1) + from + (n ? (row & 63) * kRow : 0);
-                const uint32_t at  = Lines::step(to, it);
-                cp_async16(at, src, n);
-                cp_async16(at + kPfTile / 2, src + 128, n);
-            }
-            asm volatile("cp.async.commit_group;" ::: "memory");
-            return;
-        }
 #pragma unroll
         for (int it = 0; it < kIter; ++it) {
             if (w + kPfLoaders * it >= kInstr) {
@@ -230,6 +209,33 @@ struct PrefillRows: PrefillRowMap<KVBITS> {
                 sts128(tile + prefill_offset(c0 + k, key), r[0], r[1], r[2], r[3]);
             }
         }
+    }
+};
+
+// ... T rows (PrefillLineMap), straight into the operand tile `dst`
+template<class T>
+struct PrefillRows<T, 16> {
+    using Map = PrefillLineMap;
+    static constexpr int kRow = kPfD * 2;
+
+    B200_DEVICE void fetch(const PrefillParams& p, const PrefillKeyTile& x, int is_v, uint32_t dst, int w, int lane)
+    {
+        const uint32_t to   = dst + Map::place(w, lane);
+        const int64_t  from = is_v * p.block_len * kRow + Map::unit0(lane) * 16;
+        const int      last = x.last - x.j * kPfKeys;
+#pragma unroll
+        for (int it = 0; it < Map::kIter; ++it) {
+            const int row = Map::row_of(w, lane, it);
+            if (it + 1 == Map::kIter && !Map::inside(w, it)) {
+                break;
+            }
+            const int      n   = row <= last ? 16 : 0;
+            const char*    src = (Map::row_of(w, 0, it) < 64 ? x.data0 : x.data1) + from + (n ? (row & 63) * kRow : 0);
+            const uint32_t at  = Map::step(to, it);
+            cp_async16(at, src, n);
+            cp_async16(at + kPfTile / 2, src + 128, n);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
     }
 };
 
@@ -297,7 +303,7 @@ B200_DEVICE float max3(float a, float b, float c)
 }
 
 // SPLIT: p.partial is there; else whole pieces (a kernel of its own: both walks in one cost registers, 181 -> 194 us on the
-// prompts above)
+// prompts above).  The split form is at its 128 registers and spills 40 bytes, the whole one does not spill.
 template<class T, int KVBITS, bool SPLIT>
 __global__ void __launch_bounds__(kPfThreads, 1) prefill_attention_kernel(const PrefillParams p)
 {
@@ -365,7 +371,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attention_kernel(const 
             to.find(p, Rows::kRow);
             return true;
         };
-        // A piece's Q tiles [d/8][row][8], fetched behind its first keys: the earlier piece's last softmax is under way then
+        // A piece's Q tiles, fetched behind its first keys: the earlier piece's last softmax is under way then
         PrefillQueries queries;
         bool           first = true;
         uint32_t       phq   = 1;
@@ -724,8 +730,9 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_attention_kernel(const 
 
 // Combines the partials of every (unit, kv-head) whose keys fell into several CTAs.  grid (CTA, 2 tiles, 4 x 32 dims): the block of
 // the first CTA whose range begins inside the piece does the work; thread = row and 16 of the 32 dims, parts in CTA order.
-// 16 dims a thread, so that all blocks are resident at once (with 8 dims and twice the blocks prompts take 2 us more, 4 x 400 - 512 tokens behind 300 -
-// 1000 keys 95.8 instead of 94.0, 8 x 16 behind 3000 - 4000 56.4 instead of 54.6; 32 dims: 141, 95.3 and 54.3)
+// 16 dims a thread: with 8 dims and twice the blocks, each of which looks its piece up and reads the maxima and sums of all parts again, prompts take 2 us more,
+// 4 x 400 - 512 tokens behind 300 - 1000 keys 95.8 instead of 94.0, 8 x 16 behind 3000 - 4000 56.4 instead of 54.6 (32 dims: 141, 95.3 and 54.3).  Registers
+// go from 72 to 109, resident blocks from three to two per SM: four fillings of the SMs for 148 ranges, where it was five.
 constexpr int kPfMergeThreads = 256, kPfMergeZ = 4;
 
 template<class T>

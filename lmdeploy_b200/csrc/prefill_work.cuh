@@ -207,20 +207,19 @@ B200_HD bool prefill_parts(const PrefillParams& p, int first, PrefillParts& x)
     return x.cf + 1 == first;  // else an earlier CTA has it
 }
 
-// Loader warps: the 16-byte units of 128 token rows of K or of V.  A warp instruction takes 8 rows x 4 units (64 contiguous bytes per
-// row); the 8 lanes that store one 8-dim chunk write 128 contiguous bytes of the operand tile (no bank conflicts).
+// Loader warps: the 16-byte units of 128 quantised token rows of K or of V.  A warp instruction takes 8 rows x 4 units (64 contiguous bytes per
+// row); the 8 lanes that store one 8-dim chunk of as many rows write to eight places of a line's width (prefill_offset: no bank conflicts).
 template<int KVBITS>
 struct PrefillRowMap {
+    static_assert(KVBITS == 8 || KVBITS == 4, "T rows: PrefillLineMap");
     static constexpr int kRow   = kPfD * KVBITS / 8;
-    static constexpr int kUnits = kRow / 16;                               // 16 / 8 / 4 per row
+    static constexpr int kUnits = kRow / 16;                               // 8 / 4 per row
     static constexpr int kInstr = kPfKeys / 8 * (kUnits / 4);              // warp instructions per tile
-    static constexpr int kIter  = (kInstr + kPfLoaders - 1) / kPfLoaders;  // 10 / 5 / 3 per warp
+    static constexpr int kIter  = (kInstr + kPfLoaders - 1) / kPfLoaders;  // 5 / 3 per warp
 
     B200_HD static int key_of(int w, int lane, int it) { return (w + kPfLoaders * it) / (kUnits / 4) * 8 + (lane & 7); }
     B200_HD static int unit_of(int w, int lane, int it) { return (w + kPfLoaders * it) % (kUnits / 4) * 4 + (lane >> 3); }
     B200_HD static int half_of(int w, int it) { return (w + kPfLoaders * it) / (kUnits / 4) >> 3; }  // warp-uniform: key >> 6
-    // bytes of the operand tile [d / 8][key][8]: 8 dims of a key
-    B200_HD static int chunk_offset(int chunk, int key) { return chunk * (kPfKeys * 16) + key * 16; }
 };
 
 // Operand tiles of Q, K and V: two halves of 64 dims, in each a row of 128 bytes per token whose 16-byte chunks are permuted by the row's last three

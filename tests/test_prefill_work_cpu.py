@@ -1,7 +1,7 @@
 """How prefill attention cuts and deals out its work (csrc/prefill_work.cuh, the header that the kernels compile), by a host compiler: over many ragged
 batches, grids and GQA groups every key tile of every (sequence block, kv-head) is walked exactly once, the parts of a piece that CTAs share lie in the
-slots that the merge reads, each by one CTA, and the form without room for partials walks the same pieces whole.  Also the loader warps' map: every
-16-byte unit of a tile once, eight lanes of a store side by side."""
+slots that the merge reads, each by one CTA, and the form without room for partials walks the same pieces whole.  Also the loader warps' map of
+quantised rows: every 16-byte unit of a tile once, every chunk of the operand tile once, eight lanes of a store in different banks."""
 import os
 import subprocess
 
@@ -112,7 +112,7 @@ template<int KVBITS>
 static void rows()
 {
     using M = PrefillRowMap<KVBITS>;
-    std::set<int> units;
+    std::set<int> units, places;
     for (int w = 0; w < kPfLoaders; ++w)
         for (int it = 0; it < M::kIter; ++it) {
             if (w + kPfLoaders * it >= M::kInstr) break;
@@ -120,18 +120,25 @@ static void rows()
                 const int key = M::key_of(w, lane, it), unit = M::unit_of(w, lane, it);
                 CHECK(key >= 0 && key < kPfKeys && unit >= 0 && unit < M::kUnits && M::half_of(w, it) == key / 64);
                 CHECK(units.insert(key * M::kUnits + unit).second);
-                if (lane % 8) CHECK(M::chunk_offset(unit, key) == M::chunk_offset(M::unit_of(w, lane - 1, it), M::key_of(w, lane - 1, it)) + 16);
+                for (int k = 0; k < 16 / KVBITS; ++k) CHECK(places.insert(prefill_offset(unit * (16 / KVBITS) + k, key)).second);
             }
+            for (int k = 0; k < 16 / KVBITS; ++k)        // eight lanes store at once, each to 16 bytes of its own among the 32 banks
+                for (int group = 0; group < 4; ++group) {
+                    std::set<int> banks;
+                    for (int lane = 8 * group; lane < 8 * group + 8; ++lane)
+                        banks.insert(prefill_offset(M::unit_of(w, lane, it) * (16 / KVBITS) + k, M::key_of(w, lane, it)) / 16 % 8);
+                    CHECK(banks.size() == 8);
+                }
         }
-    CHECK((int)units.size() == kPfKeys * M::kUnits);
-    CHECK(M::chunk_offset(kPfD / 8 - 1, kPfKeys - 1) + 16 == kPfKeys * kPfD * 2);
+    CHECK((int)units.size() == kPfKeys * M::kUnits && (int)places.size() == kPfKeys * kPfD / 8);
+    CHECK(*places.begin() == 0 && *places.rbegin() + 16 == kPfKeys * kPfD * 2);
 }
 
 int main(int argc, char** argv)
 {
     std::mt19937 rng(std::atoi(argv[1]));
     auto pick = [&](int n) { return (int)(rng() % n); };
-    rows<16>(), rows<8>(), rows<4>();
+    rows<8>(), rows<4>();
     const int heads[][2] = {{32, 8}, {48, 8}, {64, 8}, {28, 4}, {16, 8}, {8, 2}, {7, 1}, {2, 2}, {128, 1}, {3, 1}, {100, 1}};
     const int edges[] = {0, 1, 2, 63, 64, 65, 127, 128, 129, 255, 256, 257, 383, 384};
     for (int i = 0; i < 4000; ++i) {
