@@ -469,8 +469,9 @@ struct ThinShape {
 //         2 tiles: 4096 x 14336 17.0 / 18.0; 19.8 / 20.0, 1024 x 32768 11.4 / 10.9; 12.9 / 11.7, 4096 x 22016 29.6 / 20.7; 35.5 / 26.3
 //         3 tiles: 5120 x 5120 13.1 / 14.2; 14.9 / 15.9, 8192 x 3072 14.9 / 13.1; 16.1 / 14.4, 4096 x 8192 12.1 / 14.8; 13.4 / 15.7, 2048 x
 //         16384 13.0 / 11.6; 14.2 / 12.9
-//         (the lines were drawn when the tcgen05 kernel took 2 - 8 us more, seven conversions a pair; one tile of 75 - 132 M weights in f16 and of 75 - 84 M
-//         in bf16 would be better off there now)
+//         The lines are older than these figures (the tcgen05 kernel took 2 - 8 us more, seven conversions a pair) and no longer lie where the two meet: one tile
+//         of 75 - 132 M weights in f16 and of 75 - 84 M in bf16, and three tiles of short K (2048 x 16384), would be better off on the tcgen05 kernel, by up to 24 %.
+//         A line that moves gives the shapes between another order of sums
 //   dense 1 tile:  8192 x 1024 9.6 / 10.3, 14336 x 1024 14.9 / 12.2, 14336 x 4096 20.2 / 25.7, 4096 x 32000 40.4 / 43.6, 8192 x 10240 30.6 / 28.4 (12 SMs have two
 //         CTAs, the others one), 4096 x 46336 69 / 61
 //         2 tiles: 4096 x 4096 9.8 / 12.4, 3072 x 6144 12.9 / 13.0, 8192 x 2048 15.1 / 12.5, 5120 x 5120 19.4 / 15.2

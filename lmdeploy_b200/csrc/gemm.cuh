@@ -190,20 +190,6 @@ B200_DEVICE uint32_t e4m3x2_to(uint32_t x)  // two e4m3 bytes (low half of x) ->
     return h2;
 }
 
-// the T product of the tcgen05 kernel's weights: exact, rounded once
-template<class T>
-B200_DEVICE uint32_t mul2(uint32_t a, uint32_t b)
-{
-    uint32_t d;
-    if constexpr (std::is_same<T, nv_bfloat16>::value) {
-        asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    }
-    else {
-        asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    }
-    return d;
-}
-
 template<class T>
 B200_DEVICE void store_out(const Params& p, int tok, int col, float v)
 {
@@ -642,8 +628,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const Params p)
 #pragma unroll
                             for (int x = 0; x < 4; ++x) {
                                 const uint32_t w4    = (&v[q][u].x)[x];
-                                r[u * 8 + x * 2]     = mul2<T>(e4m3x2_to<T>(w4 & 0xffffu), sc);
-                                r[u * 8 + x * 2 + 1] = mul2<T>(e4m3x2_to<T>(w4 >> 16), sc);
+                                r[u * 8 + x * 2]     = Ops::mul2(e4m3x2_to<T>(w4 & 0xffffu), sc);
+                                r[u * 8 + x * 2 + 1] = Ops::mul2(e4m3x2_to<T>(w4 >> 16), sc);
                             }
                         }
                     }

@@ -171,8 +171,8 @@ __global__ void __launch_bounds__(kThinThreads, 2) linear_thin_kernel(const Para
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
                         const uint32_t q0 = w[st][r][i >> 1][(i & 1) * 2 + (e >> 1)], q1 = w[st][r][i >> 1][4 + (i & 1) * 2 + (e >> 1)];
-                        a0[e] = mul2<T>(e4m3x2_to<T>(e & 1 ? q0 >> 16 : q0 & 0xffffu), s0);
-                        a1[e] = mul2<T>(e4m3x2_to<T>(e & 1 ? q1 >> 16 : q1 & 0xffffu), s1);
+                        a0[e] = Ops::mul2(e4m3x2_to<T>(e & 1 ? q0 >> 16 : q0 & 0xffffu), s0);
+                        a1[e] = Ops::mul2(e4m3x2_to<T>(e & 1 ? q1 >> 16 : q1 & 0xffffu), s1);
                     }
                 }
 #pragma unroll
